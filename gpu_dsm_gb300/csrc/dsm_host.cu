@@ -197,6 +197,26 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) {
   return DSM_OK;
 }
 
+// Monodisperse equilibrium ensembles that run in the lockstep kernel
+// (dsm_lockstep.cu) rather than in tiles of 16 lanes.  It pays where most events
+// are slides, which it does four lanes to a chain, eight chains to a warp; the
+// creations and destructions, a larger share the shorter the chains and their
+// strands (small beta), go through service warps one chain at a time.  Measured
+// (events/s, lockstep against tiles; p = 64, m = 8 where G(t)):
+//   beta 1    N_K  75 2.56e9 / 2.54e9   N_K 100 3.14e9 / 2.66e9   N_K 200 3.56e9 / 2.59e9
+//     G(t)    N_K 100 1.83e9 / 1.84e9   N_K 130 2.30e9 / 2.13e9   N_K 200 2.79e9 / 2.25e9
+//   beta 0.5  N_K 100 2.04e9 / 2.28e9   N_K 150 2.58e9 / 2.31e9
+//     G(t)    N_K 150 1.98e9 / 2.03e9   N_K 463 2.18e9 / 1.08e9
+//   beta 2    N_K 100 3.51e9 / 2.85e9   N_K 300 3.17e9 / 2.24e9
+//     G(t)    N_K 100 1.94e9 / 2.00e9   N_K 150 2.54e9 / 2.19e9
+// (default_schedule adds: more chains than the tiles hold at once.)  Strand
+// sizes and the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
+static bool prefer_lock(const dsm_sim* s) {
+  const dsm_params& P = s->P;
+  if (P.lanes_per_chain != 0 || s->flow || s->poly || s->nkmax >= 16384) return false;
+  return (double)P.nk >= (s->corr ? 125.0 : 80.0) * (2.0 + 1.0 / (double)P.beta) / 3.0;
+}
+
 int dsm::sim_setup(dsm_sim* s) {
   dsm_params& P = s->P;
   if (P.nk < 1 || P.n_chains < 1 || !(P.beta > 0.0f)) return fail(s, DSM_ERR_INVALID, "invalid nk / n_chains / beta");
@@ -266,6 +286,8 @@ int dsm::sim_setup(dsm_sim* s) {
   const size_t n = (size_t)P.n_chains, cap = (size_t)s->cap;
   size_t need = n * cap * (16 + 4) + n * sizeof(ChainState) + n * 8 * 4;
   if (s->corr) need += n * s->levels * ((size_t)s->cp * (12 + 8) + 12 + 16);
+  const size_t kahan_bytes = s->corr && prefer_lock(s) ? n * ((size_t)s->cp * sizeof(float2) + 3 * kCorrBuf * sizeof(float)) : 0;
+  need += kahan_bytes;
   size_t fre = 0, tot = 0;
   CK(cudaMemGetInfo(&fre, &tot));
   if (need + (64ull << 20) > fre) return fail(s, DSM_ERR_MEMORY, "ensemble needs " + std::to_string(need >> 20) + " MiB of device memory, " + std::to_string(fre >> 20) + " MiB free");
@@ -365,6 +387,12 @@ int dsm::sim_setup(dsm_sim* s) {
     const int rc = s->poly ? plan_classes(s, 0, 0, 0, 0.f) : default_schedule(s);
     if (rc != DSM_OK) return rc;
   }
+  if (s->cfg.lock && s->corr) {
+    CK(cudaMallocAsync((void**)&s->d_ccomp, n * s->cp * sizeof(float2), s->st));
+    CK(cudaMallocAsync((void**)&s->d_cbuf, n * 3 * kCorrBuf * sizeof(float), s->st));
+    s->h.corr_comp = s->d_ccomp;  // (every launch copies the descriptor)
+    s->h.corr_buf = s->d_cbuf;
+  }
   CK(cudaStreamSynchronize(s->st));  // host-side sources of the copies above
   s->ready = true;
   return DSM_OK;
@@ -384,8 +412,39 @@ static int largest_slot(bool flow, int corr, LaunchCfg cfg, int bps_want, int hi
 
 // Fewer warps per block while the block's slots exceed the per-block shared
 // memory (long chains: one warp per block holds one slot of z_max strands)
-static void fit_block(LaunchCfg& cfg, int optin) {
-  while (cfg.warps_per_block > 1 && step_block_smem(cfg) > (size_t)optin) cfg.warps_per_block /= 2;
+static void fit_block(bool flow, LaunchCfg& cfg, int optin) {
+  while (cfg.warps_per_block > 1 && step_block_smem(flow, cfg) > (size_t)optin) cfg.warps_per_block /= 2;
+}
+
+// Slots per block of a lockstep launch over n chains: as many as fit 6 blocks
+// per SM when that is a full block (and the kernel has a build for it), else as
+// many as fit 4; fewer when that spreads the chains over equal waves.  Returns
+// the blocks per SM the choice is made for (0: not a lockstep launch).
+static int plan_lock(const dsm_sim* s, LaunchCfg& c, long long n) {
+  c.tiles = 0;
+  if (!c.lock || s->flow || lock_lanes(c.slot_cap) == 0) return 0;
+  int sm_bytes = 0, reserved = 0;
+  cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->P.device);
+  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, s->P.device);
+  const int most = 64 / lock_lanes(c.slot_cap);  // two slide warps per block
+  auto fits = [&](int blocks) {
+    int t = most;
+    while (t > 0 && (lock_block_bytes(c.slot_cap, t) + reserved) * blocks > (size_t)sm_bytes) --t;
+    return t;
+  };
+  int bps = 6, t = fits(6);
+  if (t < most || s->ck != 0) {
+    bps = 4;
+    t = fits(4);
+  }
+  if (t < 1) {
+    c.lock = false;
+    return 0;
+  }
+  // equal waves: a last wave with few chains would leave most slots empty
+  const long long blocks = (long long)bps * s->sm_count, waves = (n + blocks * t - 1) / (blocks * t);
+  c.tiles = (int)std::max<long long>(1, (n + blocks * waves - 1) / (blocks * waves));
+  return bps;
 }
 
 // One launch over all chains with slots of the full capacity
@@ -395,15 +454,16 @@ static int plan_single(dsm_sim* s) {
   s->cfg.slot_cap = s->cap;
   int smem_optin = 0;
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->P.device));
-  fit_block(s->cfg, smem_optin);
-  if (step_block_smem(s->cfg) > (size_t)smem_optin)
+  const int lock_bps = plan_lock(s, s->cfg, s->P.n_chains);
+  if (lock_bps == 0) fit_block(s->flow, s->cfg, smem_optin);
+  if (step_block_smem(s->flow, s->cfg) > (size_t)smem_optin)
     return fail(s, DSM_ERR_INVALID, "chain capacity z_max=" + std::to_string(s->cap) + " does not fit one shared-memory slot");
   const int bps = step_max_blocks_per_sm(s->flow, s->ck, s->cfg);
   if (bps < 1) return fail(s, DSM_ERR_CUDA, "step kernel cannot be resident (occupancy 0)");
-  s->blocks_per_sm = bps;
-  const int tiles = s->cfg.warps_per_block * 32 / s->cfg.lanes;
+  s->blocks_per_sm = lock_bps > 0 ? std::min(bps, lock_bps) : bps;
+  const int tiles = step_tiles(s->flow, s->cfg);
   const long long want = ((long long)s->P.n_chains + tiles - 1) / tiles;
-  s->grid = (int)std::min<long long>(want, (long long)bps * s->sm_count);
+  s->grid = (int)std::min<long long>(want, (long long)s->blocks_per_sm * s->sm_count);
   return DSM_OK;
 }
 
@@ -456,10 +516,8 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
     else { huge.push_back(i); nk_huge = std::max(nk_huge, nk); }
   }
   auto by_nk = [&](int a, int b) { return s->nk_chain[a] != s->nk_chain[b] ? s->nk_chain[a] > s->nk_chain[b] : a < b; };
-  std::sort(huge.begin(), huge.end(), by_nk);
-  std::sort(big.begin(), big.end(), by_nk);
-  std::sort(mid.begin(), mid.end(), by_nk);
-  std::sort(small.begin(), small.end(), by_nk);
+  if (s->poly)  // (chains of one length are in order already)
+    for (std::vector<int>* v : {&huge, &big, &mid, &small}) std::sort(v->begin(), v->end(), by_nk);
   std::vector<int> order(huge);
   order.insert(order.end(), big.begin(), big.end());
   order.insert(order.end(), mid.begin(), mid.end());
@@ -507,20 +565,25 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
     // with the small one for block slots, and a work-share grid left it
     // finishing alone at the end of every window (measured 9.6e8 vs 1.2e9
     // events/s on the 262144-chain log-normal melt)
-    M.cfg = LaunchCfg{4, mid_cap, s->cfg.pmax, 32};
+    M.cfg = LaunchCfg{4, mid_cap, s->cfg.pmax, 32, s->cfg.lock};
+    const int lb = plan_lock(s, M.cfg, (long long)mid.size());
     M.bps = step_max_blocks_per_sm(s->flow, s->ck, M.cfg);
+    if (lb > 0) M.bps = std::min(M.bps, lb);
     if (M.bps < 1) return fail(s, DSM_ERR_INVALID, "middle slot does not fit shared memory");
     M.first = H.count + B.count;
+    const int mt = step_tiles(s->flow, M.cfg);
     M.count = (long long)mid.size();
-    M.grid = (int)std::max<long long>(1, std::min<long long>((M.count + 3) / 4, (long long)M.bps * s->sm_count));
+    M.grid = (int)std::max<long long>(1, std::min<long long>((M.count + mt - 1) / mt, (long long)M.bps * s->sm_count));
   }
-  Sm.cfg = LaunchCfg{4, small_cap, s->cfg.pmax, sc.lanes};
+  Sm.cfg = LaunchCfg{4, small_cap, s->cfg.pmax, sc.lanes, s->cfg.lock};
+  const int small_lb = plan_lock(s, Sm.cfg, (long long)small.size());
   Sm.bps = step_max_blocks_per_sm(s->flow, s->ck, Sm.cfg);
+  if (small_lb > 0) Sm.bps = std::min(Sm.bps, small_lb);
   if (Sm.bps < 1) return fail(s, DSM_ERR_INVALID, "small slot does not fit shared memory");
   Sm.first = H.count + B.count + M.count;
   Sm.count = (long long)small.size();
   {
-    const int tiles = 4 * 32 / Sm.cfg.lanes;
+    const int tiles = step_tiles(s->flow, Sm.cfg);
     Sm.grid = (int)std::max<long long>(1, std::min<long long>((Sm.count + tiles - 1) / tiles,
                                                                 (long long)Sm.bps * s->sm_count));
   }
@@ -538,7 +601,8 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
   if (s->carve && !s->flow && sc.lanes == 16) {
     LaunchCfg full = sc;
     full.slot_cap = full_cap;
-    plan_carve(s, B, M, Sm, step_block_smem(full));
+    full.lock = false;
+    plan_carve(s, B, M, Sm, step_block_smem(false, full));
   }
   return DSM_OK;
 }
@@ -597,7 +661,7 @@ extern "C" void dsm_destroy(dsm_sim* s) {
   if (s->side2) cudaStreamSynchronize(s->side2);
   if (s->side3) cudaStreamSynchronize(s->side3);
   void* ptrs[] = {s->d_tables, s->d_QN, s->d_tau, s->d_cs, s->d_stress, s->d_cshift, s->d_cacc, s->d_cavg,
-                  s->d_ccnt, s->d_gsum, s->d_gcnt, s->d_pcd_by_nk, s->d_nk_chain, s->d_ens, s->d_prefix,
+                  s->d_ccnt, s->d_ccomp, s->d_cbuf, s->d_gsum, s->d_gcnt, s->d_pcd_by_nk, s->d_nk_chain, s->d_ens, s->d_prefix,
                   s->d_work, s->d_status, s->d_counters, s->d_red, s->d_order, s->d_defer, s->d_works, s->d_gex};
   // stream-ordered frees: no device-wide synchronisation
   for (void* p : ptrs) if (p) cudaFreeAsync(p, s->st);
@@ -625,8 +689,7 @@ extern "C" const char* dsm_last_error(const dsm_sim* s) { return s ? s->err.c_st
 // with G(t), +24 % for shear at N_K = 100).  A chain that still outgrows the
 // slot finishes in the overflow launch.  Otherwise one warp per chain with
 // full-capacity slots.
-static int default_schedule(dsm_sim* s) {
-  if (s->P.lanes_per_chain != 0) return plan_single(s);
+static int tile_schedule(dsm_sim* s) {
   LaunchCfg c = s->cfg;
   c.lanes = 16;
   c.warps_per_block = 4;
@@ -656,12 +719,33 @@ static int default_schedule(dsm_sim* s) {
   return plan_single(s);
 }
 
+// Tiles, or the lockstep kernel where it is the faster one (prefer_lock) and the
+// chains are more than the tiles hold at once: with fewer, the tiles' shorter
+// latency per event wins (N_K = 200 with G(t), 4864 of them resident: 4864 chains
+// 1.86e9 events/s against 2.32e9 in tiles, 6080 chains 2.21e9 against 1.67e9).
+// Its slot is the smallest that holds the chains' bound, so that as many chains as
+// possible are resident.
+static int default_schedule(dsm_sim* s) {
+  if (s->P.lanes_per_chain != 0) return plan_single(s);
+  const int rc = tile_schedule(s);
+  if (rc != DSM_OK || !prefer_lock(s)) return rc;
+  const LaunchCfg& t = s->classes.empty() ? s->cfg : s->classes.back().cfg;
+  if ((long long)s->P.n_chains <= (long long)s->blocks_per_sm * s->sm_count * step_tiles(s->flow, t)) return rc;
+  const double pe = 1.0 / (1.0 + (double)s->P.beta), nk = (double)s->P.nk;
+  const double zb = 1.0 + (nk - 1.0) * pe + 5.0 * std::sqrt(std::max(0.0, (nk - 1.0) * pe * (1.0 - pe))) + 2.0;
+  const int slot = std::max(8, (int)std::ceil(zb));
+  if (lock_lanes(std::min(slot, s->cap)) == 0) return rc;
+  s->cfg.lanes = 16;
+  s->cfg.lock = true;
+  return slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
+}
+
 extern "C" int dsm_set_schedule(dsm_sim* s, int32_t small_slot, int32_t large_grid, int32_t lanes,
                                 float z_margin_sd) {
   if (!s || !s->ready) return DSM_ERR_INVALID;
   if (lanes != 0 && lanes != 16 && lanes != 32) return fail(s, DSM_ERR_INVALID, "lanes must be 16 or 32");
   CK(cudaStreamSynchronize(s->st));
-  if (lanes) s->cfg.lanes = lanes;
+  if (lanes) { s->cfg.lanes = lanes; s->cfg.lock = false; }
   // monodisperse ensembles keep one launch with full-capacity slots unless a
   // smaller slot is asked for (chains that outgrow it finish in the overflow launch)
   if (!s->poly && small_slot <= 0) return plan_single(s);
@@ -1183,6 +1267,13 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   return DSM_OK;
 }
 
+// Status word of a launch: bit 0 aborted through the run flag, bit 1 a wait
+// between the warps of a block ran out
+static int launch_status(dsm_sim* s, int status) {
+  if (status & 2) return fail(s, DSM_ERR_CUDA, "step kernel: a wait between warps ran out");
+  return (status & 1) ? DSM_ABORTED : DSM_OK;
+}
+
 static void stress_out(const double* r, dsm_stress_plus* o) {
   const double d = r[8] > 0 ? r[8] : 1.0;
   o->xx = (float)(r[0] / d); o->yy = (float)(r[1] / d); o->zz = (float)(r[2] / d);
@@ -1204,8 +1295,7 @@ static int series_collect(dsm_sim* s, dsm_stress_plus* out, uint64_t* events) {
     for (int q = 0; q < 9; ++q) s->hw->red[q] = h_out[9 * (n - 1) + q];
     if (out) for (int w = 0; w < n; ++w) stress_out(h_out + 9 * w, &out[w]);
   }
-  if (s->hw->status & 1) return DSM_ABORTED;
-  return DSM_OK;
+  return launch_status(s, s->hw->status);
 }
 
 // wait for the pending work of s, forwarding the caller's abort flag
@@ -1332,8 +1422,7 @@ static int window_collect(dsm_sim* s, uint64_t* events) {
   s->t_done = std::max(s->t_done, s->t_window);
   s->last_events = cnt[0];
   CK(cudaEventElapsedTime(&s->last_kernel_ms, s->ev0, s->ev1));
-  if (status & 1) return DSM_ABORTED;
-  return DSM_OK;
+  return launch_status(s, status);
 }
 
 int dsm::sim_finish_window(dsm_sim* s, uint64_t* events) {
@@ -1505,6 +1594,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
     bool flow;
     int corr;  // correlator kind (0 none, 1 stress, 2 MSD)
     int cap_class, cp, lanes;
+    bool lock;
   };
   auto cap_class = [](int cap) { int c = 16; while (c < cap) c <<= 1; return c; };
   std::vector<Group> groups;
@@ -1512,10 +1602,11 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
     const bool fl = sims[i]->flow;
     const int co = sims[i]->ck;
     const int cc = cap_class(sims[i]->cap), cp = co ? sims[i]->cp : 0, ln = sims[i]->cfg.lanes;
+    const bool lk = sims[i]->cfg.lock;
     Group* g = nullptr;
     for (auto& x : groups)
-      if (x.flow == fl && x.corr == co && x.cap_class == cc && x.cp == cp && x.lanes == ln) g = &x;
-    if (!g) { groups.push_back(Group{{}, fl, co, cc, cp, ln}); g = &groups.back(); }
+      if (x.flow == fl && x.corr == co && x.cap_class == cc && x.cp == cp && x.lanes == ln && x.lock == lk) g = &x;
+    if (!g) { groups.push_back(Group{{}, fl, co, cc, cp, ln, lk}); g = &groups.back(); }
     g->idx.push_back(i);
   }
   // windows of every ensemble (same bookkeeping as dsm_advance)
@@ -1542,6 +1633,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   std::vector<cudaStream_t> used;
   cudaEvent_t ready = nullptr;
   std::vector<cudaEvent_t> joins;
+  std::vector<std::pair<int, int*>> words;  // first ensemble of a group, its launch's status word
   const bool fan = groups.size() > 1;
   auto enqueue = [&]() -> int {
     if (fan) {
@@ -1552,7 +1644,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       const int k = (int)g.idx.size();
       std::vector<EnsDev> hE(k);
       std::vector<long long> pre(k + 1, 0);
-      LaunchCfg cfg{4, 0, 0, g.lanes};
+      LaunchCfg cfg{4, 0, 0, g.lanes, g.lock};
       cudaStream_t gs = fan ? sims[g.idx[0]]->st : s->st;
       for (int q = 0; q < k; ++q) {
         dsm_sim* x = sims[g.idx[q]];
@@ -1590,10 +1682,12 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       const bool overflow = all_small && small < cfg.slot_cap;
       LaunchCfg run = cfg;
       if (overflow) run.slot_cap = small;
-      fit_block(run, optin);
-      const int bps = step_max_blocks_per_sm(g.flow, g.corr, run);
+      const int lock_bps = plan_lock(sims[g.idx[0]], run, pre[k]);
+      if (lock_bps == 0) fit_block(g.flow, run, optin);
+      int bps = step_max_blocks_per_sm(g.flow, g.corr, run);
       if (bps < 1) return fail(s, DSM_ERR_INVALID, "batch slot does not fit shared memory");
-      const int tiles = run.warps_per_block * 32 / run.lanes;
+      if (lock_bps > 0) bps = std::min(bps, lock_bps);
+      const int tiles = step_tiles(g.flow, run);
       const long long want = (pre[k] + tiles - 1) / tiles;
       const int grid = (int)std::min<long long>(want, (long long)bps * s->sm_count);
       StepList lst;
@@ -1614,6 +1708,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
         CK(cudaStreamWaitEvent(gs, ready, 0));
       }
       used.push_back(gs);
+      words.push_back({g.idx[0], (int*)(dW + 1)});
       CK(launch_step(dE, k, dP, pre[k], dW, g.flow, g.corr, run, nullptr, (int*)(dW + 1), grid, gs, lst));
       if (overflow) {
         StepList ol;
@@ -1637,6 +1732,8 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       }
       CK(cudaMemcpyAsync(q->hw->cnt, q->d_counters, sizeof(q->hw->cnt), cudaMemcpyDeviceToHost, s->st));
     }
+    for (const auto& w : words)
+      CK(cudaMemcpyAsync(&sims[w.first]->hw->status, w.second, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     return DSM_OK;
   };
   const int rc = enqueue();
@@ -1652,6 +1749,8 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   if (sync_err != cudaSuccess)
     return fail(s, DSM_ERR_CUDA, std::string("dsm_advance_batch: ") + cudaGetErrorString(sync_err));
   CK(cudaGetLastError());
+  for (const auto& w : words)
+    if (const int st = launch_status(s, sims[w.first]->hw->status)) return st;
   for (int i = 0; i < n; ++i) {
     const unsigned long long* cnt = sims[i]->hw->cnt;
     if (events) events[i] = cnt[0];

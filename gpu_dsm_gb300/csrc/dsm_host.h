@@ -102,6 +102,8 @@ struct dsm_sim {
   double* d_cacc = nullptr;
   float* d_cavg = nullptr;
   int4* d_ccnt = nullptr;
+  float2* d_ccomp = nullptr;  // level-0 compensated sums of a running launch
+  float* d_cbuf = nullptr;    // samples of the lockstep kernel not yet correlated
   double* d_gsum = nullptr;
   long long* d_gcnt = nullptr;
   dsm::PcdDev* d_pcd_by_nk = nullptr;

@@ -84,6 +84,8 @@ struct EnsDev {
   double* corr_acc;
   float* corr_avg;
   int4* corr_cnt;
+  float2* corr_comp;               // [chain][p] compensated level-0 sums of the running launch
+  float* corr_buf;                 // [chain][kCorrBuf][3] samples of the running launch not yet correlated
   float* out_stress;               // [chain][8] stress at the end of the launch (flow)
   unsigned long long* counters;    // [0] events this launch, [1] chains done
   // flow output series inside one launch (n_win > 0): window w ends at
@@ -95,6 +97,7 @@ struct EnsDev {
   int32_t n_win, win_stride;
 };
 
+constexpr int kCorrBuf = 64;  // samples of a chain that the lockstep kernel correlates at a time
 constexpr int kCarveMax = 4;  // size classes of one carved launch
 
 struct LaunchCfg {
@@ -102,9 +105,19 @@ struct LaunchCfg {
   int slot_cap;        // strands per SMEM slot (max cap of the ensembles launched)
   int pmax;            // correlator points per level (max over ensembles)
   int lanes = 32;      // lanes per chain: 32 (one chain per warp) or 16 (two per warp)
+  // equilibrium: the slots run by the lockstep kernel where it is built for the
+  // slot size, `tiles` of them per block (0: warps_per_block * 32 / lanes)
+  bool lock = false;
+  int tiles = 0;
 };
 
 __host__ __device__ size_t step_slot_bytes(int slot_cap, int pmax);
+// lockstep kernel (dsm_lockstep.cu): lanes per chain at a slot size (0: not built
+// for it), shared memory of a block of `tiles` slots, and the kernel of a
+// correlator kind (hi: the build for 6 blocks per SM)
+int lock_lanes(int slot_cap);
+size_t lock_block_bytes(int slot_cap, int tiles);
+void* lock_kernel(int ck, int slot_cap, bool hi);
 
 // Work list of one step launch.  Items are order[0 .. n) (global chain ids
 // across the launched ensembles; order == NULL: the identity over [0, total)),
@@ -155,7 +168,9 @@ cudaError_t launch_step(const EnsDev* d_ens, int n_ens, const long long* d_prefi
                         const StepList& lst = StepList{});
 // corr: correlator kind, 0 none, 1 stress G(t), 2 centre-of-mass MSD
 int step_max_blocks_per_sm(bool flow, int corr, const LaunchCfg& cfg);
-size_t step_block_smem(const LaunchCfg& cfg);
+size_t step_block_smem(bool flow, const LaunchCfg& cfg);
+// slots of a block
+int step_tiles(bool flow, const LaunchCfg& cfg);
 cudaError_t launch_gt_reduce_dev(const EnsDev* d_ens, int levels, int p, double* d_gsum, long long* d_count,
                                  cudaStream_t st);
 cudaError_t launch_window_begin(EnsDev* d_ens, const long long* d_win, int n, int w, cudaStream_t st);
