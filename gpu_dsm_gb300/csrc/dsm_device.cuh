@@ -171,6 +171,25 @@ struct Corr0 {  // correlator level-0 counters of the resident chain
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// ---- time slices (EnsDev::subs)
+// End of slice `sub` of a launch window
+__device__ __forceinline__ long long slice_end(const EnsDev& E, int sub) {
+  const long long a = E.t_begin_ticks, b = E.t_end_ticks;
+  return (sub + 1 >= E.subs || b <= a) ? b : a + (b - a) / E.subs * (sub + 1);
+}
+// Slices of the chain that are done; what the SM that ran the last one wrote is
+// visible after it (by every lane that synchronises with this one)
+__device__ __forceinline__ unsigned slices_done(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// (one lane, after the chain's lanes have synchronised on their stores)
+__device__ __forceinline__ void slices_set(unsigned* p, unsigned v) {
+  __threadfence();
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 // Position of a CD creation inside a strand of N1 Kuhn steps
 // (ensemble_kernel.cu:386: newn = floor(0.5 + pr (N1 - 2) / w) + 1) on the
 // quantised values r < w: x = floor((2 r (N1 - 2) + w) / (2 w)), exactly.  An

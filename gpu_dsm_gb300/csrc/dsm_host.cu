@@ -360,6 +360,7 @@ int dsm::sim_setup(dsm_sim* s) {
   E.dt_sample_ticks = s->corr ? (int64_t)std::llrint(P.sync_dt * TICKS) : 0;
   E.nsamples = s->nsamples;
   E.t_end_ticks = 0; E.step_limit = INT64_MAX; E.watchdog_events = INT64_MAX;
+  E.subs = 1;
   E.pcd = s->pcd.dev;
   E.pcd_by_nk = s->d_pcd_by_nk; E.nk_chain = s->d_nk_chain;
   if (P.pd_flag != 0) {
@@ -387,12 +388,6 @@ int dsm::sim_setup(dsm_sim* s) {
     const int rc = s->poly ? plan_classes(s, 0, 0, 0, 0.f) : default_schedule(s);
     if (rc != DSM_OK) return rc;
   }
-  if (s->cfg.lock && s->corr) {
-    CK(cudaMallocAsync((void**)&s->d_ccomp, n * s->cp * sizeof(float2), s->st));
-    CK(cudaMallocAsync((void**)&s->d_cbuf, n * 3 * kCorrBuf * sizeof(float), s->st));
-    s->h.corr_comp = s->d_ccomp;  // (every launch copies the descriptor)
-    s->h.corr_buf = s->d_cbuf;
-  }
   CK(cudaStreamSynchronize(s->st));  // host-side sources of the copies above
   s->ready = true;
   return DSM_OK;
@@ -418,7 +413,7 @@ static void fit_block(bool flow, LaunchCfg& cfg, int optin) {
 
 // Slots per block of a lockstep launch over n chains: as many as fit 6 blocks
 // per SM when that is a full block (and the kernel has a build for it), else as
-// many as fit 4; fewer when that spreads the chains over equal waves.  Returns
+// many as fit 4; with few chains no more than spread them over all SMs.  Returns
 // the blocks per SM the choice is made for (0: not a lockstep launch).
 static int plan_lock(const dsm_sim* s, LaunchCfg& c, long long n) {
   c.tiles = 0;
@@ -441,10 +436,63 @@ static int plan_lock(const dsm_sim* s, LaunchCfg& c, long long n) {
     c.lock = false;
     return 0;
   }
-  // equal waves: a last wave with few chains would leave most slots empty
-  const long long blocks = (long long)bps * s->sm_count, waves = (n + blocks * t - 1) / (blocks * t);
-  c.tiles = (int)std::max<long long>(1, (n + blocks * waves - 1) / (blocks * waves));
+  const long long blocks = (long long)bps * s->sm_count;
+  c.tiles = (int)std::max<long long>(1, std::min<long long>(t, (n + blocks - 1) / blocks));
   return bps;
+}
+
+// Time slices for n chains on `slots` slots.  A chain is a serial job, so n chains
+// in one piece take ceil(n / slots) rounds, the last of them with most slots
+// empty; cut into K slices each, worked off slice by slice, they take
+// ceil(n K / slots) / K.  Only for slots of 8 lanes per chain (lock_slices),
+// whose few chains per SM leave its issue slots idle in the last round (G(t), 50
+// tau: 4096 chains of N_K=463, beta 0.5, 3648 slots 14.1 -> 11.6 ms; 6000 of
+// N_K=300 on 4864 slots 11.2 -> 9.3; 5000 of N_K=400, beta 1, 10.3 -> 8.4), at 3
+// or 4 slices; 6 or 8 gain nothing more and cost up to 6 %.  With 4 lanes per
+// chain the other chains of the SM run the faster in the last round, and the
+// chains of a block leave and enter their slots at the same time, which keeps its
+// two service warps busy for as long: 16384 chains of N_K=200 12.7 ms either way,
+// 11000 of N_K=150 8.2 ms whole and 11.0 in two slices.
+static int slices_for(long long n, long long slots) {
+  if (slots < 1 || n <= slots) return 1;
+  int best = 1;
+  double cost = 1e300;
+  for (int k = 1; k <= 4; ++k) {
+    const double c = (double)((n * k + slots - 1) / slots) / k * (1.0 + 0.02 * (k - 1));
+    if (c < cost * 0.99) {
+      cost = c;
+      best = k;
+    }
+  }
+  return best;
+}
+
+// Per-chain buffers of the lockstep plan: time slices, and the level-0 sums and
+// samples that the kernel keeps in HBM
+static int plan_buffers(dsm_sim* s) {
+  const size_t n = s->P.n_chains;
+  const LaunchCfg& c = s->classes.empty() ? s->cfg : s->classes.back().cfg;
+  const long long items = s->classes.empty() ? (long long)n : s->classes.back().count;
+  const int grid = s->classes.empty() ? s->grid : s->classes.back().grid;
+  s->sub_max = c.lock && s->classes.size() <= 1 && lock_slices(c.slot_cap) ? slices_for(items, (long long)grid * step_tiles(s->flow, c)) : 1;
+  if (s->sub_max > 1 && !s->d_slice) CK(cudaMallocAsync((void**)&s->d_slice, n * sizeof(Slice), s->st));
+  if (s->corr && c.lock && !s->d_ccomp) {
+    CK(cudaMallocAsync((void**)&s->d_ccomp, n * s->cp * sizeof(float2), s->st));
+    CK(cudaMallocAsync((void**)&s->d_cbuf, n * 3 * kCorrBuf * sizeof(float), s->st));
+  }
+  // (every launch copies the descriptor)
+  s->h.slice = s->d_slice;
+  s->h.corr_comp = s->d_ccomp;
+  s->h.corr_buf = s->d_cbuf;
+  return DSM_OK;
+}
+
+// Slices of a launch whose shortest window is dt_tau: a slice of at least about
+// 500 events per chain; none under an event limit (it counts events, not time)
+static int launch_slices(const dsm_sim* s, double dt_tau, int64_t step_limit) {
+  if (s->sub_max <= 1 || step_limit >= 0) return 1;
+  const double ev = 0.21 * (double)s->P.nk * std::max(0.0, dt_tau);
+  return std::max(1, std::min(s->sub_max, (int)std::min(ev / 500.0, 1000.0)));
 }
 
 // One launch over all chains with slots of the full capacity
@@ -464,7 +512,7 @@ static int plan_single(dsm_sim* s) {
   const int tiles = step_tiles(s->flow, s->cfg);
   const long long want = ((long long)s->P.n_chains + tiles - 1) / tiles;
   s->grid = (int)std::min<long long>(want, (long long)s->blocks_per_sm * s->sm_count);
-  return DSM_OK;
+  return plan_buffers(s);
 }
 
 int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float margin_sd) {
@@ -604,7 +652,7 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
     full.lock = false;
     plan_carve(s, B, M, Sm, step_block_smem(false, full));
   }
-  return DSM_OK;
+  return plan_buffers(s);
 }
 
 // The carved form of a class plan: the large, middle and small classes run in
@@ -662,7 +710,7 @@ extern "C" void dsm_destroy(dsm_sim* s) {
   if (s->side3) cudaStreamSynchronize(s->side3);
   void* ptrs[] = {s->d_tables, s->d_QN, s->d_tau, s->d_cs, s->d_stress, s->d_cshift, s->d_cacc, s->d_cavg,
                   s->d_ccnt, s->d_ccomp, s->d_cbuf, s->d_gsum, s->d_gcnt, s->d_pcd_by_nk, s->d_nk_chain, s->d_ens, s->d_prefix,
-                  s->d_work, s->d_status, s->d_counters, s->d_red, s->d_order, s->d_defer, s->d_works, s->d_gex};
+                  s->d_work, s->d_status, s->d_counters, s->d_red, s->d_order, s->d_defer, s->d_works, s->d_gex, s->d_slice};
   // stream-ordered frees: no device-wide synchronisation
   for (void* p : ptrs) if (p) cudaFreeAsync(p, s->st);
   if (s->ev_fork) cudaEventDestroy(s->ev_fork);
@@ -1083,12 +1131,18 @@ static int enqueue_carved(dsm_sim* s) {
   return DSM_OK;
 }
 
+static int enqueue_slice_flush(dsm_sim* s) {
+  if (s->sub_max > 1 && s->corr) CK(launch_slice_flush(s->d_ens, s->ck, s->P.n_chains, s->st));
+  return DSM_OK;
+}
+
 static int enqueue_step(dsm_sim* s) {
+  if (s->sub_max > 1) CK(cudaMemsetAsync(s->d_slice, 0, (size_t)s->P.n_chains * sizeof(Slice), s->st));
   if (s->classes.empty()) {
     CK(cudaMemsetAsync(s->d_work, 0, sizeof(unsigned int), s->st));
     CK(launch_step(s->d_ens, 1, s->d_prefix, (long long)s->P.n_chains, s->d_work, s->flow, s->ck, s->cfg,
                    s->d_abort, s->d_status, s->grid, s->st));
-    return DSM_OK;
+    return enqueue_slice_flush(s);
   }
   CK(cudaMemsetAsync(s->d_works, 0, 16 * sizeof(unsigned int), s->st));
   const int rc = s->carved ? enqueue_carved(s) : enqueue_classes(s);
@@ -1099,7 +1153,7 @@ static int enqueue_step(dsm_sim* s) {
   l.dyn_total = s->d_works + 3;
   CK(launch_step(s->d_ens, 1, s->d_prefix, 0, s->d_works + 2, s->flow, s->ck, s->cleanup.cfg, s->d_abort,
                  s->d_status, s->cleanup.grid, s->st, l));
-  return DSM_OK;
+  return enqueue_slice_flush(s);
 }
 
 int dsm::sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit) {
@@ -1108,6 +1162,8 @@ int dsm::sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit) {
   s->t_window = t_end;
   E.step_limit = step_limit < 0 ? INT64_MAX : step_limit;
   E.watchdog_events = window_watchdog(s, t_end - s->t_done);
+  E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
+  E.subs = launch_slices(s, t_end - s->t_done, step_limit);
   CK(cudaMemcpyAsync(s->d_ens, &E, sizeof(EnsDev), cudaMemcpyHostToDevice, s->st));
   CK(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->st));
   CK(cudaMemsetAsync(s->d_counters, 0, 4 * sizeof(unsigned long long), s->st));
@@ -1247,6 +1303,7 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   if (rc != DSM_OK) return rc;
   long long* h_win = ser_win_h(s);
   t_prev = s->t_done;
+  double shortest = ends[n - 1] - t_prev;
   for (int w = 0; w < n; ++w) {
     h_win[w] = (long long)std::llrint(ends[w] * TICKS);  // as dsm_advance(ends[w])
     h_win[s->ser_cap + w] = (long long)window_watchdog(s, ends[w] - t_prev);
@@ -1256,6 +1313,8 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   s->ser_n = n;
   EnsDev& E = s->h;
   E.step_limit = INT64_MAX;
+  E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
+  E.subs = launch_slices(s, shortest, -1);
   CK(cudaMemcpyAsync(s->d_ens, &E, sizeof(EnsDev), cudaMemcpyHostToDevice, s->st));
   if (direct) {
     rc = series_enqueue(s, n, false);
@@ -1621,6 +1680,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
     const double expect = 0.25 * (double)q->nkmax * std::max(0.0, te - q->t_done) * 100.0;
     const double wd = std::max(16777216.0, std::min(expect, 9.0e18));
     E.watchdog_events = q->watchdog_events > 0 ? q->watchdog_events : (int64_t)wd;
+    E.subs = 1;
     CK(cudaMemcpyAsync(q->d_ens, &E, sizeof(EnsDev), cudaMemcpyHostToDevice, s->st));
     CK(cudaMemsetAsync(q->d_counters, 0, 4 * sizeof(unsigned long long), s->st));
   }
@@ -1661,7 +1721,6 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       CK(cudaMallocAsync((void**)&dP, sizeof(long long) * (k + 1) + 16, s->st));
       tmp.push_back(dP);
       dW = (unsigned int*)(dP + k + 1);
-      CK(cudaMemcpyAsync(dE, hE.data(), sizeof(EnsDev) * k, cudaMemcpyHostToDevice, s->st));
       CK(cudaMemcpyAsync(dP, pre.data(), sizeof(long long) * (k + 1), cudaMemcpyHostToDevice, s->st));
       CK(cudaMemsetAsync(dW, 0, 16, s->st));
       int optin = 0;
@@ -1690,6 +1749,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       const int tiles = step_tiles(g.flow, run);
       const long long want = (pre[k] + tiles - 1) / tiles;
       const int grid = (int)std::min<long long>(want, (long long)bps * s->sm_count);
+      CK(cudaMemcpyAsync(dE, hE.data(), sizeof(EnsDev) * k, cudaMemcpyHostToDevice, s->st));
       StepList lst;
       LaunchCfg oc{1, cfg.slot_cap, cfg.pmax, 32};
       int ogrid = 0;

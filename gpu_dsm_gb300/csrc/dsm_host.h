@@ -139,6 +139,10 @@ struct dsm_sim {
   dsm::StepList carve_list;
   int carve_grid = 0;
   size_t carve_smem = 0;
+  // time slices of a launch (EnsDev::subs): the most that pay for this plan, and
+  // their per-chain words
+  int sub_max = 1;
+  dsm::Slice* d_slice = nullptr;
   cudaStream_t side = nullptr, side2 = nullptr, side3 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
   int prio = 0;  // CUDA stream priority of st and side

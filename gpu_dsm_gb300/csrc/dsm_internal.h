@@ -40,6 +40,14 @@ struct ChainState {
 static_assert(sizeof(ChainState) == 64, "ChainState layout");
 
 // Everything one kernel needs to know about one ensemble (device copy).
+// A chain of a launch in time slices
+struct __align__(16) Slice {
+  unsigned long long step0;  // event counter at the start of the launch
+  unsigned int nbuf;         // samples in corr_buf
+  unsigned int done;         // slices done; kMoved: needs none any more (larger slot, abort)
+};
+constexpr unsigned kMoved = 0xffffffffu;
+
 struct EnsDev {
   int32_t n_chains, cap, nk, cd_flag;
   int32_t flow, s0, poly, corr_type;
@@ -55,6 +63,13 @@ struct EnsDev {
   int64_t t_end_ticks;       // chains stop when T >= t_end_ticks
   int64_t step_limit;        // ... or when step >= step_limit
   int64_t watchdog_events;   // max events per chain per launch (stall 5 beyond)
+  // time slices (lockstep kernel): the launch runs every chain in `subs` pieces
+  // of equal length from t_begin_ticks to t_end_ticks, all first pieces first, so
+  // that the slots stay full to the end of the launch although the chains are no
+  // multiple of them
+  int64_t t_begin_ticks;
+  int32_t subs, pad_subs_;
+  Slice* slice;              // [chain]
   PcdDev pcd;                // monodisperse partner law
   // GEX background (pd_flag = 1): partner N_K = mp/Mk * M/mp from the inverse
   // tables M (SD-created and initial entanglements) and Md (CD-created)
@@ -84,7 +99,9 @@ struct EnsDev {
   double* corr_acc;
   float* corr_avg;
   int4* corr_cnt;
-  float2* corr_comp;               // [chain][p] compensated level-0 sums of the running launch
+  // [chain][p] compensated level-0 sums of the running launch: of a chain that is
+  // between two time slices, or resident in the lockstep kernel (else zero)
+  float2* corr_comp;
   float* corr_buf;                 // [chain][kCorrBuf][3] samples of the running launch not yet correlated
   float* out_stress;               // [chain][8] stress at the end of the launch (flow)
   unsigned long long* counters;    // [0] events this launch, [1] chains done
@@ -116,6 +133,7 @@ __host__ __device__ size_t step_slot_bytes(int slot_cap, int pmax);
 // for it), shared memory of a block of `tiles` slots, and the kernel of a
 // correlator kind (hi: the build for 6 blocks per SM)
 int lock_lanes(int slot_cap);
+bool lock_slices(int slot_cap);  // launches in time slices pay for slots of this size
 size_t lock_block_bytes(int slot_cap, int tiles);
 void* lock_kernel(int ck, int slot_cap, bool hi);
 
@@ -173,6 +191,8 @@ size_t step_block_smem(bool flow, const LaunchCfg& cfg);
 int step_tiles(bool flow, const LaunchCfg& cfg);
 cudaError_t launch_gt_reduce_dev(const EnsDev* d_ens, int levels, int p, double* d_gsum, long long* d_count,
                                  cudaStream_t st);
+// after a launch in time slices: samples and sums of chains that were stopped between two slices
+cudaError_t launch_slice_flush(const EnsDev* d_ens, int ck, int n_chains, cudaStream_t st);
 cudaError_t launch_window_begin(EnsDev* d_ens, const long long* d_win, int n, int w, cudaStream_t st);
 cudaError_t launch_stress_reduce_dev(const EnsDev* d_ens, double* d_out9, cudaStream_t st);
 // stress of every chain from its state in HBM (d_out8: n_chains x 8 floats), then the reduction

@@ -1486,6 +1486,7 @@ __global__ void k_series_reduce(const EnsDev* __restrict__ ensp, double* out) {
 
 // Window w of a captured series: end time d_win[w] and event cap d_win[n+w]
 __global__ void k_window_begin(EnsDev* ens, const long long* __restrict__ d_win, int n, int w) {
+  if (w > 0) ens->t_begin_ticks = d_win[w - 1];
   ens->t_end_ticks = d_win[w];
   ens->watchdog_events = d_win[n + w];
 }

@@ -58,7 +58,8 @@ struct __align__(16) Hdr {
   int e, c, stall, cap;
   int zlim;
   float wz1;
-  long long t_end, step_lim, lim0, pad_;
+  long long t_end, step_lim, lim0;
+  int sub, pend;                 // time slice of the resident chain; item that waits for its chain, plus one
 };
 
 struct LCorr : Corr0 {
@@ -306,6 +307,35 @@ __device__ __noinline__ void lock_flush(const EnsDev& E, int c, LCorr* k0) {
   }
   if (threadIdx.x % 32 == 0) k0->nbuf = 0;
   __syncwarp();
+}
+
+// Level 0's counters and running average from HBM, and back (one lane)
+__device__ __forceinline__ void lock_corr_load(const EnsDev& E, int c, LCorr* k0) {
+  const size_t l0 = (size_t)c * E.corr_levels;
+  const int4 cn = E.corr_cnt[l0];
+  k0->ins = cn.x; k0->navg = cn.y;
+  k0->nins = ((long long)(unsigned)cn.w) << 32 | (unsigned)cn.z;
+  k0->a0 = E.corr_avg[l0 * 3 + 0]; k0->a1 = E.corr_avg[l0 * 3 + 1]; k0->a2 = E.corr_avg[l0 * 3 + 2];
+}
+__device__ __forceinline__ void lock_corr_store(const EnsDev& E, int c, const LCorr& k0) {
+  const size_t l0 = (size_t)c * E.corr_levels;
+  E.corr_cnt[l0] = make_int4(k0.ins, k0.navg, (int)(unsigned)(k0.nins & 0xffffffffll), (int)(unsigned)(k0.nins >> 32));
+  E.corr_avg[l0 * 3 + 0] = k0.a0; E.corr_avg[l0 * 3 + 1] = k0.a1; E.corr_avg[l0 * 3 + 2] = k0.a2;
+}
+
+// End of a chain's launch: the buffered samples, then the compensated level-0
+// sums into the FP64 ones (one warp)
+template <bool MSD>
+__device__ __forceinline__ void lock_corr_out(const EnsDev& E, int c, LCorr* k0) {
+  lock_flush<MSD>(E, c, k0);
+  const int p = E.corr_p;
+  const size_t l0 = (size_t)c * E.corr_levels;
+  const float2* Cacc = E.corr_comp + (size_t)c * p;
+#pragma unroll 1
+  for (int j = threadIdx.x % 32; j < p; j += 32) {
+    const float2 a = Cacc[j];
+    E.corr_acc[l0 * p + j] += (double)a.x - (double)a.y;
+  }
 }
 
 // Centre of mass of the chain (chain_com of dsm_kernels.cu in the arithmetic of
@@ -586,10 +616,11 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
 
 // Everything a chain needs before its next slide, by one service warp: the
 // requested event, due samples, the way back to HBM and the next chain, rate
-// passes, the prefix of the pair totals.
+// passes, the prefix of the pair totals.  False: the slot's next chain is not back
+// from its earlier time slice yet, ask again.
 template <int CK, int SUBS, int SB>
-__device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n_ens,
-                                           const long long* __restrict__ prefix, long long n_items,
+__device__ __forceinline__ bool lock_serve(const EnsDev* __restrict__ ens, int n_ens,
+                                           const long long* __restrict__ prefix, long long n_items, int subs,
                                            unsigned int* work, int slot_cap, const LSlot& sl, unsigned bit, Ctl* ctl,
                                            const volatile int* abort_flag, int* status, const StepList& lst) {
   constexpr bool CORR = CK != 0, MSD = CK == 2;
@@ -644,17 +675,10 @@ __device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n
                               (float)strand_n(v.w));
           wt[s] = (s < Z - 1) ? __int_as_float(v.z) : 0.0f;
         }
-        if (CORR) {
-          lock_flush<MSD>(E, c, sl.k0);
-          const int p = E.corr_p;
-          const size_t l0 = (size_t)c * E.corr_levels;
-          const float2* Cacc = E.corr_comp + (size_t)c * p;
-#pragma unroll 1
-          for (int j = lane; j < p; j += 32) {
-            const float2 a = Cacc[j];
-            E.corr_acc[l0 * p + j] += (double)a.x - (double)a.y;
-          }
-        }
+        // the chain's last time slice of the launch: else buffered samples and
+        // sums stay for the next one
+        const bool last = h.sub + 1 >= subs || deferred || aborted;
+        if (CORR && last) lock_corr_out<MSD>(E, c, sl.k0);
         if (lane == 0) {
           ChainState* cs = &E.cs[c];
           // the launch's start values are still in HBM: events done, stored scale
@@ -666,10 +690,8 @@ __device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n
           if (CORR) {
             const LCorr& k0 = *sl.k0;
             cs->k_next = k0.k_next;
-            const size_t l0 = (size_t)c * E.corr_levels;
-            E.corr_cnt[l0] = make_int4(k0.ins, k0.navg, (int)(unsigned)(k0.nins & 0xffffffffll),
-                                       (int)(unsigned)(k0.nins >> 32));
-            E.corr_avg[l0 * 3 + 0] = k0.a0; E.corr_avg[l0 * 3 + 1] = k0.a1; E.corr_avg[l0 * 3 + 2] = k0.a2;
+            lock_corr_store(E, c, k0);
+            if (!last) E.slice[c].nbuf = (unsigned)k0.nbuf;
             if (MSD) { cs->r1[0] = k0.r1x; cs->r1[1] = k0.r1y; cs->r1[2] = k0.r1z; }
           }
           atomicAdd(&E.counters[0], done);
@@ -677,48 +699,81 @@ __device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n
           if (deferred) {
             lst.defer[atomicAdd(lst.n_defer, 1u)] = (int)(prefix[e] + c);
             atomicAdd(&E.counters[2], 1ull);
-          } else {
+          } else if (last) {
             atomicAdd(&E.counters[1], 1ull);
           }
         }
         live = false;
         __syncwarp();
+        if (subs > 1 && lane == 0) slices_set(&E.slice[c].done, deferred || aborted ? kMoved : (unsigned)h.sub + 1u);
       }
     }
     if (!live) {  // the next chain of the work list
       unsigned int item = 0;
-      if (lane == 0) item = atomicAdd(work, 1u);
+      if (lane == 0) {
+        item = h.pend != 0 ? (unsigned)h.pend - 1u : atomicAdd(work, 1u);
+        h.pend = 0;
+      }
       item = wshfl(item, 0);
-      const bool stop = (long long)item < n_items && abort_flag != nullptr && wshfl(*abort_flag, 0) != 0;
-      if ((long long)item >= n_items || stop) {
+      const bool none = (long long)item >= n_items * subs;
+      const bool stop = !none && abort_flag != nullptr && wshfl(*abort_flag, 0) != 0;
+      if (none || stop) {
         if (lane == 0) {
           if (stop) atomicOr(status, 1);
           h.Z = 0;
           atomicOr(&ctl->dead, bit);
         }
-        return;
+        return true;
       }
-      const long long gid = lst.order != nullptr ? (long long)lst.order[item] : (long long)item;
+      int sub = 0;
+      unsigned int idx = item;
+      if (subs > 1) {
+        sub = (int)(item / (unsigned)n_items);
+        idx -= (unsigned)sub * (unsigned)n_items;
+      }
+      const long long gid = lst.order != nullptr ? (long long)lst.order[idx] : (long long)idx;
       e = 0;
 #pragma unroll 1
       while (e + 1 < n_ens && prefix[e + 1] <= gid) ++e;
       const EnsDev& E = ens[e];
       c = (int)(gid - prefix[e]);
+      if (sub > 0) {
+        // the chain's earlier slice: a slot of this block may be running it, so
+        // the request is posted again instead of waiting here
+        const unsigned done = wshfl(slices_done(&E.slice[c].done), 0);
+        __syncwarp();
+        if (done < (unsigned)sub) {
+          if (lane == 0) {
+            h.pend = (int)item + 1;
+            h.rq = RQ_LOAD;
+          }
+          return false;
+        }
+        if (done == kMoved) continue;
+      }
       const ChainState st = E.cs[c];
       if (st.Z > slot_cap) {  // does not fit at all: hand it to a larger slot
         if (lane == 0) {
           lst.defer[atomicAdd(lst.n_defer, 1u)] = (int)gid;
           atomicAdd(&E.counters[2], 1ull);
+          if (subs > 1) slices_set(&E.slice[c].done, kMoved);
         }
         continue;
       }
       cap = E.cap;
       zlim = cap > slot_cap ? slot_cap : 0x7fffffff;
       Z = st.Z; S = st.S; stall = st.stall; T = st.T; step = st.step; hash = st.hash;
-      t_end = E.t_end_ticks;
+      t_end = sub + 1 < subs ? slice_end(E, sub) : E.t_end_ticks;
       lim0 = E.step_limit;
+      // (the event cap counts from the start of the launch)
       const long long wd = E.watchdog_events;
-      step_lim = (wd < lim0 - (long long)step) ? (long long)step + wd : lim0;
+      long long first = (long long)step;
+      if (subs > 1) {
+        if (sub > 0) first = (long long)E.slice[c].step0;
+        else if (lane == 0) E.slice[c].step0 = step;
+      }
+      step_lim = (wd < lim0 - first) ? first + wd : lim0;
+      if (lane == 0) h.sub = sub;
       wz1 = __double2float_rn(__ddiv_rn(1.0, __dmul_rn(E.beta_d, (double)st.nk)));
       const size_t ecap = (size_t)cap;
       const float4* gq = E.QN + (size_t)c * ecap;
@@ -735,16 +790,14 @@ __device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n
       if (CORR) {
         const int p = E.corr_p;
         float2* Cacc = E.corr_comp + (size_t)c * p;
+        if (sub == 0) {
 #pragma unroll 1
-        for (int j = lane; j < p; j += 32) Cacc[j] = make_float2(0.f, 0.f);
+          for (int j = lane; j < p; j += 32) Cacc[j] = make_float2(0.f, 0.f);
+        }
         if (lane == 0) {
-          const size_t l0 = (size_t)c * E.corr_levels;
-          const int4 cn = E.corr_cnt[l0];
           LCorr& k0 = *sl.k0;
-          k0.ins = cn.x; k0.navg = cn.y;
-          k0.nins = ((long long)(unsigned)cn.w) << 32 | (unsigned)cn.z;
-          k0.a0 = E.corr_avg[l0 * 3 + 0]; k0.a1 = E.corr_avg[l0 * 3 + 1]; k0.a2 = E.corr_avg[l0 * 3 + 2];
-          k0.nbuf = 0;  // samples in the buffer
+          lock_corr_load(E, c, &k0);
+          k0.nbuf = sub == 0 ? 0 : E.slice[c].nbuf;
           k0.k_next = st.k_next;
           k0.t_next = st.k_next * E.dt_sample_ticks;
           if (MSD) { k0.r1x = st.r1[0]; k0.r1y = st.r1[1]; k0.r1z = st.r1[2]; }
@@ -814,6 +867,28 @@ __device__ __forceinline__ void lock_serve(const EnsDev* __restrict__ ens, int n
       h.t_end = t_end; h.step_lim = step_lim; h.lim0 = lim0;
     }
   }
+  return true;
+}
+
+// After a launch in time slices: a chain that an abort stopped between two of
+// them still has its samples and sums of this launch.  One warp per chain.
+template <bool MSD>
+__global__ void __launch_bounds__(128) k_slice_flush(const EnsDev* __restrict__ ensp, int n_chains) {
+  __shared__ LCorr k0s[4];
+  const EnsDev& E = *ensp;
+  const int c = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (E.subs <= 1 || c >= n_chains) return;
+  const unsigned done = E.slice[c].done;
+  if (done == 0 || done >= (unsigned)E.subs) return;
+  LCorr* k0 = &k0s[threadIdx.x / 32];
+  if (lane == 0) {
+    lock_corr_load(E, c, k0);
+    k0->nbuf = E.slice[c].nbuf;
+  }
+  __syncwarp();
+  lock_corr_out<MSD>(E, c, k0);
+  __syncwarp();
+  if (lane == 0) lock_corr_store(E, c, *k0);
 }
 
 constexpr unsigned kSpinLimit = 1u << 28;  // polls of a wait before it gives up (status bit 1)
@@ -840,6 +915,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
       if (threadIdx.x == 0) {
         s.h->rq = RQ_LOAD;
         s.h->e = 0;
+        s.h->pend = 0;
       }
     }
     if (threadIdx.x == 0) { ctl->req = all; ctl->done = 0u; ctl->dead = 0u; ctl->served = 0u; }
@@ -849,13 +925,18 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
   if (warp >= slides) {
     // ------------------------------------------------ service warp
     const long long n_items = lst.dyn_total != nullptr ? (long long)*lst.dyn_total : total;
-    unsigned idle = 0, seen = 0;
-      for (;;) {
+    const int subs = lst.dyn_total != nullptr ? 1 : ens[0].subs;  // time slices
+    unsigned idle = 0, seen = 0, waits = 0, turn = ~0u;
+    for (;;) {
       int b = -1;
       if (lane == 0) {
         const unsigned q = *(volatile unsigned*)&ctl->req;
         if (q != 0u) {
-          b = __ffs(q) - 1;
+          // in turn: a slot that polls for its chain's earlier time slice must not
+          // keep the slot that runs it from being served
+          const unsigned next = q & turn;
+          b = __ffs(next != 0u ? next : q) - 1;
+          turn = b == 31 ? ~0u : ~0u << (b + 1);
           if ((atomicAnd(&ctl->req, ~(1u << b)) >> b & 1u) == 0u) b = -2;  // another warp took it
         } else if (*(volatile unsigned*)&ctl->dead == all) {
           b = -3;
@@ -880,13 +961,20 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
       idle = 0;
       __threadfence_block();
       const LSlot sl = lock_slot(slots + (size_t)b * sbytes, slot_cap, SB);
-      lock_serve<CK, SUBS, SB>(ens, n_ens, prefix, n_items, work, slot_cap, sl, 1u << b, ctl, abort_flag, status, lst);
+      const bool done = lock_serve<CK, SUBS, SB>(ens, n_ens, prefix, n_items, subs, work, slot_cap, sl, 1u << b, ctl,
+                                                 abort_flag, status, lst);
       __syncwarp();
       if (lane == 0) {
-        atomicAdd(&ctl->served, 1u);
+        if (done) atomicAdd(&ctl->served, 1u);
         __threadfence_block();
-        atomicOr(&ctl->done, 1u << b);
+        atomicOr(done ? &ctl->done : &ctl->req, 1u << b);
       }
+      waits = done ? 0u : waits + 1u;
+      if (waits > kSpinLimit) {
+        if (lane == 0) atomicOr(status, 2);
+        return;
+      }
+      if (!done) __nanosleep(1000);
     }
   }
 
@@ -1132,6 +1220,7 @@ static LockShape lock_shape(int slot_cap) {
   return {0, 0};
 }
 int lock_lanes(int slot_cap) { return lock_shape(slot_cap).lanes; }
+bool lock_slices(int slot_cap) { return lock_shape(slot_cap).lanes == 8; }
 size_t lock_block_bytes(int slot_cap, int tiles) {
   const LockShape f = lock_shape(slot_cap);
   return sizeof(Ctl) + lock_bytes(slot_cap, 4 * f.lanes, f.sb) * tiles;
@@ -1153,6 +1242,13 @@ void* lock_kernel(int ck, int slot_cap, bool hi) {
   const LockShape f = lock_shape(slot_cap);
   if (hi) return ck == 0 ? lock_pick<0, 6>(f) : nullptr;
   return ck == 0 ? lock_pick<0, 4>(f) : ck == 2 ? lock_pick<2, 4>(f) : lock_pick<1, 4>(f);
+}
+
+cudaError_t launch_slice_flush(const EnsDev* d_ens, int ck, int n_chains, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((n_chains + 3) / 4);
+  if (ck == 2) k_slice_flush<true><<<blocks, 128, 0, st>>>(d_ens, n_chains);
+  else k_slice_flush<false><<<blocks, 128, 0, st>>>(d_ens, n_chains);
+  return cudaGetLastError();
 }
 
 }  // namespace dsm

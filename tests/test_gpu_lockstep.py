@@ -3,6 +3,8 @@ oracle and against the 16-lane tiles, bit for bit: every built slot size (pairs
 per sub-chunk of the pick and lanes per chain), capacity refusals, CD off, the GEX
 background, both correlator kinds across several sample buffers, chains that
 outgrow their slot, and an abort."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -80,3 +82,65 @@ def test_lockstep_overflow_and_abort(dsm_mod, oracle_mod, eq_type):
     assert_bitexact(gpu_state(g), o.get_state(), what="lockstep overflow")
     assert g.advance(50.0, abort=np.ones(1, np.int32)) == -1
     assert_bitexact(gpu_state(g), o.get_state(), what="lockstep abort")
+
+
+@pytest.mark.parametrize("kw", [dict(nk=300, beta=0.5, eq_type=0),
+                                dict(nk=300, beta=0.5, eq_type=1, corr_p=64, corr_m=8),
+                                dict(nk=200, beta=0.4, eq_type=2, corr_p=16, corr_m=2),
+                                dict(nk=300, beta=0.5, eq_type=1, corr_p=64, corr_m=8, small_slot=206)], ids=str)
+def test_lockstep_time_slices(dsm_mod, kw):
+    """Launches in time slices (8 lanes per chain, more chains than slots, windows of
+    thousands of events) against the tiles: windows with and without slices, between
+    samples and with part-filled sample buffers, a series of windows, and chains that
+    outgrow their slot."""
+    kw = dict(kw)
+    small = kw.pop("small_slot", 0)
+    n = 6000
+    a = dsm_mod.Ensemble(n_chains=n, seed=74, sync_dt=0.75, t_end=4000.0, **kw)
+    b = dsm_mod.Ensemble(n_chains=n, seed=74, sync_dt=0.75, t_end=4000.0, lanes_per_chain=16, **kw)
+    if small:
+        a.set_schedule(small_slot=small, z_margin_sd=0.01)
+    for x in (a, b):
+        x.init_equilibrium()
+    deferred = 0
+    for t in (55.0, 56.0, 112.25):
+        assert a.advance(t) == b.advance(t)
+        deferred += a.window_stats()["deferred"]
+    assert (deferred > 0) == (small > 0)
+    a.advance_series(55.0, 2)
+    for t in (167.25, 222.25):
+        b.advance(t)
+    if kw["eq_type"] != 0:
+        ga, ca = a.gt_raw()
+        gb, cb = b.gt_raw()
+        assert np.array_equal(ca, cb)
+        if small:  # a sum cut in two FP32 pieces where the chain changed its slot
+            assert np.abs(ga - gb).max() <= 2.0**-22 * np.abs(gb).max()
+        else:
+            assert np.array_equal(ga, gb)
+    assert_bitexact(gpu_state(a), gpu_state(b), what=f"slices {kw}")
+
+
+def test_lockstep_abort_between_slices(dsm_mod):
+    """A launch in time slices told to abort while it runs, then run to its end:
+    no sample is lost (level-0 sums are cut in two FP32 pieces there)."""
+    kw = dict(nk=300, beta=0.5, n_chains=6000, seed=75, eq_type=1, corr_p=64, corr_m=8, sync_dt=1.0, t_end=4000.0)
+    a = dsm_mod.Ensemble(**kw)
+    b = dsm_mod.Ensemble(lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    flag = np.zeros(1, np.int32)
+
+    def stop():
+        flag[0] = 1
+    timer = threading.Timer(0.1, stop)
+    timer.start()
+    a.advance(1500.0, abort=flag)
+    timer.join()
+    a.advance(1500.0)
+    b.advance(1500.0)
+    ga, ca = a.gt_raw()
+    gb, cb = b.gt_raw()
+    assert np.array_equal(ca, cb)
+    assert np.abs(ga - gb).max() <= 2.0**-22 * np.abs(gb).max()
+    assert_bitexact(gpu_state(a), gpu_state(b), what="abort between slices")
