@@ -247,6 +247,29 @@ __device__ __forceinline__ void move_strands_down(Slot& sl, int lo, int lo_p, in
   t.sync();
 }
 
+// Whole strands from lo on move one place up (dir 1) or down (-1): Q and N over
+// [lo, Z), the pair arrays T, R and P over [lo, Z - 1).  All arrays of a lane's
+// strand are loaded before the tile synchronises and stored after it, ordered as
+// above.
+template <int W>
+__device__ __forceinline__ void move_strands(Slot& sl, int lo, int Z, int dir, const Tile<W>& t) {
+#pragma unroll 1
+  for (int done = 0; done < Z - lo; done += W) {
+    const int s = dir > 0 ? Z - 1 - done - t.lane : lo + done + t.lane;
+    const bool act = s >= lo && s < Z, pr = act && s < Z - 1;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    int n = 0;
+    float ta = 0.f;
+    unsigned long long r = 0, p = 0;
+    if (act) { q = sl.Q[s]; n = sl.N[s]; }
+    if (pr) { ta = sl.T[s]; r = sl.R[s]; p = sl.P[s]; }
+    t.sync();
+    if (act) { sl.Q[s + dir] = q; sl.N[s + dir] = n; }
+    if (pr) { sl.T[s + dir] = ta; sl.R[s + dir] = r; sl.P[s + dir] = p; }
+  }
+  t.sync();
+}
+
 // float components {CD destruction, shift +1, shift -1, CD creation} of pair p
 // (ensemble_kernel.cu:149-181,304-414)
 __device__ __forceinline__ void pair_floats(const EnsDev& E, const Slot& sl, int p, float o[4]) {
@@ -462,6 +485,7 @@ __device__ __forceinline__ void corr_push_levels(const EnsDev& E, int c, float w
     t.sync();
     if (lane == 0) { sh[ins * 3 + 0] = w0; sh[ins * 3 + 1] = w1; sh[ins * 3 + 2] = w2; }
     t.sync();
+#pragma unroll 1
     for (int j = dmin + lane; j < p; j += W) {
       if ((long long)j >= nins) break;
       int i2 = ins - j;
@@ -544,6 +568,7 @@ __device__ __forceinline__ void corr_samples(const EnsDev& E, Slot& sl, int Z, i
       chain_com<W>(E, sl, Z, c, t, v);
     } else {
       float sxy = 0.f, syz = 0.f, sxz = 0.f;
+#pragma unroll 1
       for (int s = lane; t.strand_sum_lane() && s < Z; s += 16) {
         const float4 q = sl.Q[s];
         const float w = __ldg(&E.INV3N[sl.N[s]]);
@@ -558,6 +583,7 @@ __device__ __forceinline__ void corr_samples(const EnsDev& E, Slot& sl, int Z, i
     t.sync();
     if (lane == 0) { sl.Csh[ins * 3 + 0] = v[0]; sl.Csh[ins * 3 + 1] = v[1]; sl.Csh[ins * 3 + 2] = v[2]; }
     t.sync();
+#pragma unroll 1
     for (int j = lane; j < p; j += W) {
       if ((long long)j >= n0) break;
       int i2 = ins - j;
@@ -608,7 +634,11 @@ __device__ __forceinline__ void corr_samples(const EnsDev& E, Slot& sl, int Z, i
   }
 }
 
-// ------------------------------------------------------------------ creation events
+// ------------------------------------------------------------------ creations, destructions
+// Flow has a function for each kind of structural event: its event loop, mostly
+// the rate pass, waits for instructions in 2 % of its stalls either way, and the
+// common path of apply_struct costs it 4 % more instructions (shear at N_K = 100:
+// 1.53 ms a window against 1.49).
 // Apply a creation (CD inside strand j / CD at the tail / SD at head or tail):
 // returns newn and the pairs to recompute (up0, upn).
 template <int W>
@@ -689,10 +719,9 @@ __device__ DSM_APPLY_ATTR int apply_create(const EnsDev& E, Slot& sl, int evn, i
 
 // Apply a destruction (CD of pair j, SD at head or tail): sets the pairs to
 // recompute (up0, upn).
-template <int W, bool MSD>
+template <int W>
 __device__ DSM_APPLY_ATTR void apply_destroy(Slot& sl, int evn, int j, int Z, const Tile<W> t, int* up0_out,
                                           int* upn_out) {
-  constexpr bool msd = MSD;
   const int lane = t.lane;
   if (evn == CDD) {  // ensemble_kernel.cu:312-323
     const int n = sl.N[j] + sl.N[j + 1];
@@ -707,23 +736,14 @@ __device__ DSM_APPLY_ATTR void apply_destroy(Slot& sl, int evn, int j, int Z, co
     move_strands_down(sl, j + 2, j + 1, Z, t);
     if (lane == 0) {
       sl.N[j] = n; sl.Q[j] = qm;
-      if (msd && j == 0) {  // the first entanglement is now the old second one (eq_ensemble_kernel.cu:447-455)
-        Corr0& k0 = *sl.k0;
-        k0.r1x = __fadd_rn(k0.r1x, b.x); k0.r1y = __fadd_rn(k0.r1y, b.y); k0.r1z = __fadd_rn(k0.r1z, b.z);
-      }
     }
     *up0_out = j - 1; *upn_out = 2;
   } else if (evn == SDD_HEAD) {  // ensemble_kernel.cu:492-494
     const int n = sl.N[1] + 1;
-    const float4 b = sl.Q[1];
     t.sync();
     move_strands_down(sl, 1, 1, Z, t);
     if (lane == 0) {
       sl.N[0] = n; sl.Q[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (msd) {  // eq_ensemble_kernel.cu:645-653
-        Corr0& k0 = *sl.k0;
-        k0.r1x = __fadd_rn(k0.r1x, b.x); k0.r1y = __fadd_rn(k0.r1y, b.y); k0.r1z = __fadd_rn(k0.r1z, b.z);
-      }
     }
     *up0_out = 0; *upn_out = 1;
   } else {  // SDD_TAIL, ensemble_kernel.cu:495-498
@@ -732,6 +752,134 @@ __device__ DSM_APPLY_ATTR void apply_destroy(Slot& sl, int evn, int j, int Z, co
     *up0_out = Z - 3; *upn_out = 1;
   }
   t.sync();
+}
+
+// Random words; with a correlator out of line (one copy of the code; without one
+// the call costs more than it saves, 1.41 against 1.37 ms at N_K = 100)
+__device__ __noinline__ U4 words_call(const EnsDev& E, uint32_t purpose, uint64_t ctr, int c) {
+  return rng_at(E, purpose, ctr, (uint32_t)(ctr >> 32), (uint32_t)c);
+}
+template <bool CORR>
+__device__ __forceinline__ U4 tile_words(const EnsDev& E, uint32_t purpose, uint64_t ctr, int c) {
+  return CORR ? words_call(E, purpose, ctr, c) : rng_at(E, purpose, ctr, (uint32_t)(ctr >> 32), (uint32_t)c);
+}
+
+// Apply a creation (CD inside strand j / CD at the tail / SD at head or tail,
+// ensemble_kernel.cu:380-478) or a destruction (CD of pair j, SD at head or tail,
+// :312-323,492-498).  Returns a creation's split position and the pairs to
+// recompute (up0, upn).
+// For equilibrium, whose code (samples and their levels, the slide, seven kinds of
+// structural events) was 20 KB more than the 32 KB that an SM fetches without
+// delay: half of all stalls were waits for instructions with G(t) at N_K = 50, and
+// a creation took 11800 cycles.  So one path for all kinds, one copy of each
+// function in it (with a correlator the random words out of line too), and the
+// loops over strands, lags and moves not unrolled: the event loop is 28 KB.  A 40
+// tau window of 16384 chains takes 3.1 instead of 4.3 ms (N_K = 50, beta = 2, p =
+// 16, m = 2), 4.2 instead of 5.9 (N_K = 50, p = 64, m = 8), 3.6 instead of 4.0
+// without G(t), and the same at N_K = 100 (fewer structural events); MSD, 8192
+// chains of N_K = 100, 50 tau: 5.6 instead of 6.9.
+template <bool CORR, int W, bool MSD>
+__device__ DSM_APPLY_ATTR int apply_struct(const EnsDev& E, Slot& sl, int evn, int j, int Z, int c, uint64_t step,
+                                           unsigned long long rem, unsigned long long wsel, uint32_t w2, uint32_t w3,
+                                           const Tile<W> t, int* up0_out, int* upn_out) {
+  const int lane = t.lane;
+  const bool destroy = evn == CDD || evn == SDD_HEAD || evn == SDD_TAIL;
+  // strand sa (and sa + 1 of a creation) after strands lo.. have moved by dir
+  int up0, upn, dir, lo, sa, na, nb = 0, newn = 0;
+  float4 qa = make_float4(0.f, 0.f, 0.f, 0.f), qb = qa;
+  float trate = 0.f;
+  if (destroy) {
+    const bool tail = evn == SDD_TAIL;
+    sa = evn == CDD ? j : tail ? Z - 2 : 0;
+    const int n1 = sl.N[sa], n2 = sl.N[sa + 1];
+    const float4 a = sl.Q[sa], b = sl.Q[sa + 1];
+    // CDD merges strands j and j + 1; an end destruction merges the one-step end
+    // strand into its neighbour
+    na = (evn == CDD) ? n1 + n2 : (tail ? n1 : n2) + 1;
+    if (evn == CDD && j != 0 && j != Z - 2) {
+      const float x = __fadd_rn(a.x, b.x), y = __fadd_rn(a.y, b.y), z = __fadd_rn(a.z, b.z);
+      qa = make_float4(x, y, z, m_q2(x, y, z));
+    }
+    // the pair that goes is sa, its strand sa + 1: the pairs from sa + 1 and the
+    // strands from sa + 2 move down (strand sa + 1 too, into sa, which is stored after it)
+    dir = tail ? 0 : -1;
+    lo = sa + 1;
+    up0 = evn == CDD ? j - 1 : tail ? Z - 3 : 0;
+    upn = evn == CDD ? 2 : 1;
+    if (MSD && lane == 0 && ((evn == CDD && j == 0) || evn == SDD_HEAD)) {
+      // the first entanglement is now the old second one (eq_ensemble_kernel.cu:447-455,645-653)
+      Corr0& k0 = *sl.k0;
+      k0.r1x = __fadd_rn(k0.r1x, b.x); k0.r1y = __fadd_rn(k0.r1y, b.y); k0.r1z = __fadd_rn(k0.r1z, b.z);
+    }
+  } else {
+    const bool cdc = evn == CDC_MID || evn == CDC_TAIL;
+    const int sj = evn == CDC_MID ? j : evn == SDC_HEAD ? 0 : Z - 1;
+    const int N1 = sl.N[sj];
+    const float4 qo = sl.Q[sj];
+    const U4 w = tile_words<CORR>(E, P_CREATE, step, c);
+    // lanes 0 and 1 a pair of normal deviates each, lane 2 the lifetime's power
+    const PcdDev pp = partner_pcd(E, w3, cdc);
+    const float u = u01(w2);
+    const float base = cdc ? __fmaf_rn(u, pp.Adt_, pp.Ddt_) : __fmaf_rn(u, pp.At_, pp.Dt_);
+    const float lg = m_log(lane == 0 ? u01(w.x) : lane == 1 ? u01(w.z) : base);
+    float sn, cs;
+    m_sincos2pi((lane == 0 ? w.y : w.w) >> 8, &sn, &cs);
+    // (other lanes' logarithms may be positive, a slow case of the square root)
+    const float rr = __fsqrt_rn(lane < 2 ? __fmul_rn(-2.0f, lg) : 1.0f);
+    const float ga = __fmul_rn(rr, cs), gb = __fmul_rn(rr, sn);
+    const float pw = t.shfl(m_exp(__fmul_rn(cdc ? pp.Cdt_ : pp.Ct_, lg)), 2);
+    const float g0 = t.shfl(ga, 0), g1 = t.shfl(gb, 0), g2 = t.shfl(ga, 1);
+    trate = E.cd_flag ? ((u < (cdc ? pp.Bdt_ : pp.one_minus_g)) ? pw : pp.tau_d_inv) : 0.0f;
+    if (cdc) {
+      newn = split_pos(rem, wsel, N1) + 1;
+      newn = max(1, min(N1 - 1, newn));
+    }
+    const bool inner = evn == CDC_MID && j > 0;
+    const bool head = (evn == CDC_MID && j == 0) || evn == SDC_HEAD;
+    const int nn = inner ? newn : head ? (evn == SDC_HEAD ? N1 - 1 : N1 - newn) : (evn == SDC_TAIL ? N1 - 1 : newn);
+    const int nd = N1 - nn;
+    float sg = __fsqrt_rn(__fdiv_rn(inner ? (float)(newn * (N1 - newn)) : (float)nn, inner ? (float)(3 * N1) : 3.0f));
+    if (Z == 1 && evn != CDC_MID) sg = 0.0f;
+    const float x0 = __fmul_rn(g0, sg), y0 = __fmul_rn(g1, sg), z0 = __fmul_rn(g2, sg);
+    if (inner) {
+      const float ra = __fdiv_rn((float)newn, (float)N1);
+      const float x = __fmaf_rn(qo.x, ra, x0), y = __fmaf_rn(qo.y, ra, y0), z = __fmaf_rn(qo.z, ra, z0);
+      const float x2 = __fsub_rn(qo.x, x), y2 = __fsub_rn(qo.y, y), z2 = __fsub_rn(qo.z, z);
+      sa = j; na = nn; nb = nd;
+      qa = make_float4(x, y, z, m_q2(x, y, z));
+      qb = make_float4(x2, y2, z2, m_q2(x2, y2, z2));
+      dir = 1; lo = j; up0 = j - 1; upn = 3;
+    } else {
+      const float4 qn = make_float4(x0, y0, z0, m_q2(x0, y0, z0));
+      upn = 2;
+      if (head) {
+        sa = 0; na = nd; nb = nn; qb = qn;
+        dir = 1; lo = 0; up0 = 0;
+        if (MSD && lane == 0) {  // the new first entanglement (eq_ensemble_kernel.cu:531-539,606-614)
+          Corr0& k0 = *sl.k0;
+          k0.r1x = __fsub_rn(k0.r1x, x0); k0.r1y = __fsub_rn(k0.r1y, y0); k0.r1z = __fsub_rn(k0.r1z, z0);
+        }
+      } else {
+        sa = Z - 1; na = nn; nb = nd; qa = qn;
+        dir = 0; lo = Z; up0 = Z - 2;
+      }
+    }
+  }
+  t.sync();
+  if (dir != 0) move_strands(sl, lo, Z, dir, t);
+  if (lane == 0) {
+    sl.N[sa] = na;
+    sl.Q[sa] = qa;
+    if (!destroy) {
+      sl.N[sa + 1] = nb;
+      sl.Q[sa + 1] = qb;
+      sl.T[sa] = trate;
+    }
+  }
+  t.sync();
+  *up0_out = up0;
+  *upn_out = upn;
+  return newn;
 }
 
 // ------------------------------------------------------------------ phase clocks
@@ -929,7 +1077,7 @@ __global__ void __launch_bounds__(128, MB) k_step(const EnsDev* __restrict__ ens
     bool words = !FLOW;
     if (!FLOW) {
       const uint64_t ctr = (step & ~(uint64_t)(W - 1)) + (uint64_t)lane;
-      const U4 q = rng_at(E, P_EVENT, ctr, (uint32_t)(ctr >> 32), (uint32_t)c);
+      const U4 q = tile_words<CORR>(E, P_EVENT, ctr, c);
       r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
     }
     DSM_PHASE(10);  // chain load and first rate pass
@@ -1019,7 +1167,7 @@ __global__ void __launch_bounds__(128, MB) k_step(const EnsDev* __restrict__ ens
           break;
         }
         const uint64_t ctr = (step & ~(uint64_t)(W - 1)) + (uint64_t)lane;
-        const U4 q = rng_at(E, P_EVENT, ctr, (uint32_t)(ctr >> 32), (uint32_t)c);
+        const U4 q = tile_words<CORR>(E, P_EVENT, ctr, c);
         r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
         words = true;
       }
@@ -1086,31 +1234,39 @@ __global__ void __launch_bounds__(128, MB) k_step(const EnsDev* __restrict__ ens
         up0 = j - 1; upn = 3;
         slide = !((j <= 1) || (j + 1 >= Z - 2));
         dirty = slide ? 0 : 1;
-      } else if (evn == CDD || evn == SDD_HEAD || evn == SDD_TAIL) {
-        // away from both chain ends (pair 2 <= j < Z - 3) a destruction keeps
-        // what the end rates depend on (Z >= 3, the two strands at each end):
-        // their quantised values move down with the pairs, not recomputed
-        const bool mid = !FLOW && j >= 2 && j + 3 < Z;
-        unsigned long long ev = 0;
-        if (mid && lane < NEND) ev = sl.R[np + lane];
-        apply_destroy<W, MSD>(sl, evn, j, Z, t, &up0, &upn);
-        if (mid && lane < NEND) sl.R[np - 1 + lane] = ev;
-        Z -= 1;
-        dirty = mid ? 0 : 1;
-      } else if (Z >= cap) {
-        code |= (uint32_t)NULL_FLAG << 24;  // creation refused at capacity (ensemble_kernel.cu:380,423,451)
+      } else if constexpr (FLOW) {
+        if (evn == CDD || evn == SDD_HEAD || evn == SDD_TAIL) {
+          apply_destroy<W>(sl, evn, j, Z, t, &up0, &upn);
+          Z -= 1;
+        } else if (Z >= cap) {
+          code |= (uint32_t)NULL_FLAG << 24;  // creation refused at capacity (ensemble_kernel.cu:380,423,451)
+        } else {
+          const uint32_t w2 = t.shfl(r2, src);
+          const uint32_t w3 = t.shfl(r3, src);
+          const int newn = apply_create<W>(E, sl, evn, j, Z, c, step, rem, wsel, w2, w3, t, &up0, &upn);
+          Z += 1;
+          code |= (uint32_t)newn << 8;
+        }
       } else {
-        const uint32_t w2 = t.shfl(r2, src);
-        const uint32_t w3 = t.shfl(r3, src);
-        // the same for a creation inside a strand away from both ends
-        const bool mid = !FLOW && j >= 2 && j + 3 < Z;
-        unsigned long long ev = 0;
-        if (mid && lane < NEND) ev = sl.R[np + lane];
-        const int newn = apply_create<W>(E, sl, evn, j, Z, c, step, rem, wsel, w2, w3, t, &up0, &upn);
-        if (mid && lane < NEND) sl.R[np + 1 + lane] = ev;
-        Z += 1;
-        dirty = mid ? 0 : 1;
-        code |= (uint32_t)newn << 8;
+        const bool destroy = evn == CDD || evn == SDD_HEAD || evn == SDD_TAIL;
+        // away from both chain ends (pair 2 <= j < Z - 3) the event keeps what the
+        // end rates depend on (Z >= 3, the two strands at each end): their
+        // quantised values move with the pairs, not recomputed
+        const bool mid = j >= 2 && j + 3 < Z;
+        if (!destroy && Z >= cap) {
+          code |= (uint32_t)NULL_FLAG << 24;  // creation refused at capacity
+        } else {
+          const uint32_t w2 = t.shfl(r2, src);
+          const uint32_t w3 = t.shfl(r3, src);
+          unsigned long long ev = 0;
+          if (mid && lane < NEND) ev = sl.R[np + lane];
+          const int newn = apply_struct<CORR, W, MSD>(E, sl, evn, j, Z, c, step, rem, wsel, w2, w3, t, &up0, &upn);
+          const int dz = destroy ? -1 : 1;
+          if (mid && lane < NEND) sl.R[np + dz + lane] = ev;
+          Z += dz;
+          dirty = mid ? 0 : 1;
+          code |= (uint32_t)newn << 8;
+        }
       }
       t.sync();
 #ifdef DSM_PHASE_CLOCKS

@@ -518,7 +518,8 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
     const float lg = m_log(lane == 0 ? u01(gx) : lane == 1 ? u01(gz) : base);
     float sn, cs;
     m_sincos2pi((lane == 0 ? gy : gw) >> 8, &sn, &cs);
-    const float rr = __fsqrt_rn(__fmul_rn(-2.0f, lg));
+    // (other lanes' logarithms may be positive, a slow case of the square root)
+    const float rr = __fsqrt_rn(lane < 2 ? __fmul_rn(-2.0f, lg) : 1.0f);
     const float ga = __fmul_rn(rr, cs), gb = __fmul_rn(rr, sn);
     const float pw = wshfl(m_exp(__fmul_rn(cdc ? pp.Cdt_ : pp.Ct_, lg)), 2);
     const float g0 = wshfl(ga, 0), g1 = wshfl(gb, 0), g2 = wshfl(ga, 1);
