@@ -203,18 +203,20 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) {
 // creations and destructions, a larger share the shorter the chains and their
 // strands (small beta), go through service warps one chain at a time.  Measured
 // (events/s, lockstep against tiles; p = 64, m = 8 where G(t)):
-//   beta 1    N_K  75 2.56e9 / 2.54e9   N_K 100 3.14e9 / 2.66e9   N_K 200 3.56e9 / 2.59e9
-//     G(t)    N_K 100 1.83e9 / 1.84e9   N_K 130 2.30e9 / 2.13e9   N_K 200 2.79e9 / 2.25e9
-//   beta 0.5  N_K 100 2.04e9 / 2.28e9   N_K 150 2.58e9 / 2.31e9
-//     G(t)    N_K 150 1.98e9 / 2.03e9   N_K 463 2.18e9 / 1.08e9
-//   beta 2    N_K 100 3.51e9 / 2.85e9   N_K 300 3.17e9 / 2.24e9
-//     G(t)    N_K 100 1.94e9 / 2.00e9   N_K 150 2.54e9 / 2.19e9
+//   beta 1    N_K  75 2.43e9 / 2.70e9   N_K 100 2.94e9 / 2.75e9   N_K 200 3.53e9 / 2.57e9
+//     G(t)    N_K 100 1.89e9 / 2.55e9   N_K 130 2.35e9 / 2.27e9   N_K 200 2.86e9 / 2.27e9
+//     MSD     N_K 130 2.09e9 / 2.19e9   N_K 150 2.21e9 / 2.23e9   N_K 200 2.64e9 / 2.20e9
+//   beta 0.5  N_K 100 2.00e9 / 2.55e9   N_K 150 2.52e9 / 2.35e9
+//     G(t)    N_K 150 2.00e9 / 2.17e9   N_K 200 1.95e9 / 1.89e9   N_K 463 1.96e9 / 1.04e9
+//   beta 2    N_K 100 3.35e9 / 2.84e9   N_K 300 3.20e9 / 2.33e9
+//     G(t)    N_K 100 2.01e9 / 2.56e9   N_K 150 2.52e9 / 2.60e9   N_K 200 3.01e9 / 2.29e9
 // (default_schedule adds: more chains than the tiles hold at once.)  Strand
 // sizes and the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
 static bool prefer_lock(const dsm_sim* s) {
   const dsm_params& P = s->P;
   if (P.lanes_per_chain != 0 || s->flow || s->poly || s->nkmax >= 16384) return false;
-  return (double)P.nk >= (s->corr ? 125.0 : 80.0) * (2.0 + 1.0 / (double)P.beta) / 3.0;
+  const double f = (2.0 + 1.0 / (double)P.beta) / 3.0;
+  return (double)P.nk >= (s->corr ? 150.0 * std::max(1.0, f) : 100.0 * f);
 }
 
 int dsm::sim_setup(dsm_sim* s) {

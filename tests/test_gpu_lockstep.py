@@ -42,11 +42,11 @@ def test_lockstep_bitexact(dsm_mod, oracle_mod, kw):
     assert_bitexact(gpu_state(g), o.get_state(), what=f"lockstep {kw}, event limit")
 
 
-@pytest.mark.parametrize("kw", [dict(nk=131, eq_type=1, corr_p=16, corr_m=2),
+@pytest.mark.parametrize("kw", [dict(nk=151, eq_type=1, corr_p=16, corr_m=2),
                                 dict(nk=200, eq_type=1, corr_p=64, corr_m=8),
-                                dict(nk=180, beta=0.5, eq_type=1, corr_p=96, corr_m=4),
-                                dict(nk=140, eq_type=2, corr_p=64, corr_m=8),
-                                dict(nk=131, eq_type=2, corr_p=8, corr_m=2)], ids=str)
+                                dict(nk=204, beta=0.5, eq_type=1, corr_p=96, corr_m=4),
+                                dict(nk=150, eq_type=2, corr_p=64, corr_m=8),
+                                dict(nk=151, eq_type=2, corr_p=8, corr_m=2)], ids=str)
 def test_lockstep_correlator_equals_tiles(dsm_mod, kw):
     """States, G(t) or MSD sums and R1 over windows that end inside, at and after
     full sample buffers (80 and 7 samples per window)."""
@@ -67,10 +67,10 @@ def test_lockstep_correlator_equals_tiles(dsm_mod, kw):
 def test_lockstep_overflow_and_abort(dsm_mod, oracle_mod, eq_type):
     """Slots a little above the mean strand count: many chains finish in the
     overflow launch; then a launch that is told to abort before it starts."""
-    kw = dict(nk=131, n_chains=N, seed=73)
+    kw = dict(nk=151, n_chains=N, seed=73)
     g = dsm_mod.Ensemble(eq_type=eq_type, sync_dt=1.0, t_end=100.0, corr_p=16, corr_m=2, **kw)
     o = oracle_mod.Oracle(**kw)
-    g.set_schedule(small_slot=70, z_margin_sd=0.01)
+    g.set_schedule(small_slot=80, z_margin_sd=0.01)
     g.init_equilibrium()
     o.init_equilibrium()
     deferred = 0
@@ -86,7 +86,7 @@ def test_lockstep_overflow_and_abort(dsm_mod, oracle_mod, eq_type):
 
 @pytest.mark.parametrize("kw", [dict(nk=300, beta=0.5, eq_type=0),
                                 dict(nk=300, beta=0.5, eq_type=1, corr_p=64, corr_m=8),
-                                dict(nk=200, beta=0.4, eq_type=2, corr_p=16, corr_m=2),
+                                dict(nk=230, beta=0.4, eq_type=2, corr_p=16, corr_m=2),
                                 dict(nk=300, beta=0.5, eq_type=1, corr_p=64, corr_m=8, small_slot=206)], ids=str)
 def test_lockstep_time_slices(dsm_mod, kw):
     """Launches in time slices (8 lanes per chain, more chains than slots, windows of
