@@ -125,6 +125,7 @@ int dsm::corr_levels_for(double t_end, double dt, int p, int m) {
 
 static int plan_single(dsm_sim* s);
 static int default_schedule(dsm_sim* s);
+static int poly_schedule(dsm_sim* s);
 static void series_free(dsm_sim* s);
 static int enqueue_readback(dsm_sim* s);
 static int window_collect(dsm_sim* s, uint64_t* events);
@@ -387,7 +388,7 @@ int dsm::sim_setup(dsm_sim* s) {
     return fail(s, DSM_ERR_INVALID, "lanes_per_chain must be 16 or 32");
   s->cfg.lanes = P.lanes_per_chain > 0 ? P.lanes_per_chain : 32;
   {
-    const int rc = s->poly ? plan_classes(s, 0, 0, 0, 0.f) : default_schedule(s);
+    const int rc = s->poly ? poly_schedule(s) : default_schedule(s);
     if (rc != DSM_OK) return rc;
   }
   CK(cudaStreamSynchronize(s->st));  // host-side sources of the copies above
@@ -788,6 +789,33 @@ static int default_schedule(dsm_sim* s) {
   s->cfg.lanes = 16;
   s->cfg.lock = true;
   return slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
+}
+
+// Per-chain N_K.  One chain per warp has the lower latency, two per warp (16 lanes,
+// with a middle class of one per warp for the chains that outgrow its slot) the
+// higher throughput, which counts when the whole work at its 1.9e9 events/s lasts
+// longer than the longest chain at 2.2 us per event: sum N_K above 4100 times the
+// largest N_K.  A middle class between a hundredth of the chains and two full
+// rounds of its slots holds the other one up.  20 tau of G(t), 32 and 16 lanes:
+// 32768 chains, mean N_K 150, PDI 1.5 (6060 in the middle class) 12.4 and 11.2 ms;
+// 16384, 100, 1.1 (93) 4.8 and 3.5; 32768, 50, 1.1 (none) 5.0 and 4.2; but 32768,
+// 60, 2.0 (1500) 6.4 and 7.9; below the limit 32768, 60, 1.5 with N_K up to 810
+// 6.1 and 7.1, and 8192, 150, 2.0 3.7 and 4.8.
+static int poly_schedule(dsm_sim* s) {
+  double sum = 0.0;
+  for (int nk : s->nk_chain) sum += nk;
+  if (s->flow || s->P.lanes_per_chain != 0 || sum < 4100.0 * s->nkmax) return plan_classes(s, 0, 0, 0, 0.f);
+  const int lanes = s->cfg.lanes;
+  s->cfg.lanes = 16;
+  const int rc = plan_classes(s, 0, 0, 16, 0.f);
+  if (rc != DSM_OK) return rc;
+  for (const SizeClass& k : s->classes)
+    if (k.stream == 2 && k.count > s->P.n_chains / 100 &&
+        k.count < 2ll * k.bps * s->sm_count * step_tiles(s->flow, k.cfg)) {
+      s->cfg.lanes = lanes;
+      return plan_classes(s, 0, 0, 0, 0.f);
+    }
+  return rc;
 }
 
 extern "C" int dsm_set_schedule(dsm_sim* s, int32_t small_slot, int32_t large_grid, int32_t lanes,
