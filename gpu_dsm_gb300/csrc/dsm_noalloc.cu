@@ -146,13 +146,31 @@ extern "C" int dsm_advance_noalloc(const dsm_params* p, dsm_float4* d_QN, float*
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   // long chains: fewer warps (chain slots) per block until the block fits
-  while (cfg.warps_per_block > 1 && dsm::step_slot_bytes(cap, 0) * cfg.warps_per_block > (size_t)optin)
-    cfg.warps_per_block /= 2;
-  if (dsm::step_slot_bytes(cap, 0) * cfg.warps_per_block > (size_t)optin)
-    return fail(DSM_ERR_INVALID, "z_max does not fit one shared-memory slot");
-  const int bps = dsm::step_max_blocks_per_sm(flow, false, cfg);
+  auto fit = [&](int lanes) {
+    cfg.lanes = lanes;
+    cfg.warps_per_block = 4;
+    while (cfg.warps_per_block > 1 && dsm::step_block_smem(flow, cfg) > (size_t)optin) cfg.warps_per_block /= 2;
+    return dsm::step_block_smem(flow, cfg) <= (size_t)optin;
+  };
+  if (!fit(32)) return fail(DSM_ERR_INVALID, "z_max does not fit one shared-memory slot");
+  int bps = dsm::step_max_blocks_per_sm(flow, false, cfg);
   if (bps < 1) return fail(DSM_ERR_CUDA, "step kernel cannot be resident");
-  const long long want = ((long long)p->n_chains + cfg.warps_per_block - 1) / cfg.warps_per_block;
+  // Two chains per warp where that makes half as many chains again resident and
+  // the chains need more than one round of single ones and a full or two rounds of
+  // double ones (32 and 16 lanes, 8 tau: 32768 chains of N_K = 60 1.95 and 1.56 ms,
+  // N_K = 131 3.57 and 2.99, in shear 7.2 and 6.3; 3600 of N_K = 60 0.29 and 0.33;
+  // 7000 of N_K = 131, a little more than one round of 6080, 0.93 and 0.96; N_K =
+  // 300, whose slots leave no more than 18 chains per SM either way, 4.2 and 5.4).
+  const long long n = p->n_chains, r32 = (long long)bps * sms * dsm::step_tiles(flow, cfg);
+  if (n > r32) {
+    const dsm::LaunchCfg one = cfg;
+    const int b16 = fit(16) ? dsm::step_max_blocks_per_sm(flow, false, cfg) : 0;
+    const long long r16 = (long long)b16 * sms * dsm::step_tiles(flow, cfg);
+    if (2 * r16 >= 3 * r32 && (n <= r16 || n >= 2 * r16)) bps = b16;
+    else cfg = one;
+  }
+  const int tiles = dsm::step_tiles(flow, cfg);
+  const long long want = ((long long)p->n_chains + tiles - 1) / tiles;
   const int grid = (int)(want < (long long)bps * sms ? want : (long long)bps * sms);
   e = dsm::launch_step((const dsm::EnsDev*)(dbase + kOffEns), 1, (const long long*)(dbase + kOffPrefix),
                        (long long)p->n_chains, (unsigned int*)(dbase + kOffWork), flow, false, cfg, nullptr,
