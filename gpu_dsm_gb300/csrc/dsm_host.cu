@@ -126,6 +126,7 @@ int dsm::corr_levels_for(double t_end, double dt, int p, int m) {
 static int plan_single(dsm_sim* s);
 static int default_schedule(dsm_sim* s);
 static int poly_schedule(dsm_sim* s);
+static int small_schedule(dsm_sim* s);
 static void series_free(dsm_sim* s);
 static int enqueue_readback(dsm_sim* s);
 static int window_collect(dsm_sim* s, uint64_t* events);
@@ -183,10 +184,11 @@ void dsm::keep_pool_memory(int device) {
 }
 
 // ------------------------------------------------------------------ lifecycle
-extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) {
+int dsm::sim_create(const dsm_params* p, bool shared, dsm_sim** out) {
   if (!p || !out) return DSM_ERR_INVALID;
   *out = nullptr;
   dsm_sim* s = new dsm_sim();
+  s->shared = shared;
   s->P = *p;
   const int rc = dsm::sim_setup(s);
   if (rc != DSM_OK) {
@@ -197,6 +199,8 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) {
   *out = s;
   return DSM_OK;
 }
+
+extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_create(p, false, out); }
 
 // Monodisperse equilibrium ensembles that run in the lockstep kernel
 // (dsm_lockstep.cu) rather than in tiles of 16 lanes.  It pays where most events
@@ -390,6 +394,8 @@ int dsm::sim_setup(dsm_sim* s) {
   {
     const int rc = s->poly ? poly_schedule(s) : default_schedule(s);
     if (rc != DSM_OK) return rc;
+    const int rs = small_schedule(s);
+    if (rs != DSM_OK) return rs;
   }
   CK(cudaStreamSynchronize(s->st));  // host-side sources of the copies above
   s->ready = true;
@@ -791,6 +797,44 @@ static int default_schedule(dsm_sim* s) {
   return slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
 }
 
+// Blocks per SM of one launch with one chain per warp and full-capacity slots,
+// and in cfg its shape (0: does not fit)
+static int one_per_warp(bool flow, int ck, int cap, int pmax, int optin, LaunchCfg& cfg) {
+  cfg = LaunchCfg{4, cap, pmax, 32};
+  fit_block(flow, cfg, optin);
+  return step_block_smem(flow, cfg) <= (size_t)optin ? step_max_blocks_per_sm(flow, ck, cfg) : 0;
+}
+
+// Ensembles whose chains are all resident with one chain per warp run so: an event
+// of a 32-lane tile takes 0.7 of the time of a 16-lane tile's while the GPU is not
+// full.  12 tau, 32 and 16 lanes: N_K = 50, 1024 chains, G(t) 0.277 and 0.394 ms,
+// none 0.255 and 0.359, shear 0.354 and 0.462; 3648 chains (24 per SM) 0.400 and
+// 0.449, 0.380 and 0.414, 0.485 and 0.538; 4096 chains 0.507 and 0.482, 0.480 and
+// 0.429, 0.644 and 0.564.  Not where the 16-lane plan is one of 4 blocks per SM
+// (G(t) of long chains, whose larger register budget leaves little: 3648 chains of
+// N_K = 100 0.62 either way), not for MSD (as in poly_schedule), and not for
+// ensembles that share the GPU with others.
+static int small_schedule(dsm_sim* s) {
+  const dsm_params& P = s->P;
+  if (P.lanes_per_chain != 0 || s->shared || s->ck == 2 || s->poly || s->cfg.lock || s->cfg.lanes != 16 || s->blocks_per_sm < 5 ||
+      P.n_chains > 24ll * s->sm_count)
+    return DSM_OK;
+  int optin = 0;
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, P.device));
+  LaunchCfg c;
+  const int bps = one_per_warp(s->flow, s->ck, s->cap, s->cfg.pmax, optin, c);
+  if (P.n_chains > (long long)bps * s->sm_count * step_tiles(s->flow, c)) return DSM_OK;
+  s->slot16 = s->classes.empty() ? s->cap : s->classes.back().cfg.slot_cap;
+  s->cfg.lanes = 32;
+  return plan_single(s);
+}
+
+// Back to the two-per-warp widths before a schedule is asked for
+static void small_schedule_end(dsm_sim* s) {
+  if (s->slot16 > 0) s->cfg.lanes = 16;
+  s->slot16 = 0;
+}
+
 // Per-chain N_K.  One chain per warp has the lower latency, two per warp (16 lanes,
 // with a middle class of one per warp for the chains that outgrow its slot) the
 // higher throughput, which counts when the whole work at its 1.9e9 events/s lasts
@@ -800,11 +844,12 @@ static int default_schedule(dsm_sim* s) {
 // 32768 chains, mean N_K 150, PDI 1.5 (6060 in the middle class) 12.4 and 11.2 ms;
 // 16384, 100, 1.1 (93) 4.8 and 3.5; 32768, 50, 1.1 (none) 5.0 and 4.2; but 32768,
 // 60, 2.0 (1500) 6.4 and 7.9; below the limit 32768, 60, 1.5 with N_K up to 810
-// 6.1 and 7.1, and 8192, 150, 2.0 3.7 and 4.8.
+// 6.1 and 7.1, and 8192, 150, 2.0 3.7 and 4.8.  Not for MSD: the order of the
+// centre-of-mass sums follows the lanes.
 static int poly_schedule(dsm_sim* s) {
   double sum = 0.0;
   for (int nk : s->nk_chain) sum += nk;
-  if (s->flow || s->P.lanes_per_chain != 0 || sum < 4100.0 * s->nkmax) return plan_classes(s, 0, 0, 0, 0.f);
+  if (s->flow || s->ck == 2 || s->P.lanes_per_chain != 0 || sum < 4100.0 * s->nkmax) return plan_classes(s, 0, 0, 0, 0.f);
   const int lanes = s->cfg.lanes;
   s->cfg.lanes = 16;
   const int rc = plan_classes(s, 0, 0, 16, 0.f);
@@ -823,6 +868,7 @@ extern "C" int dsm_set_schedule(dsm_sim* s, int32_t small_slot, int32_t large_gr
   if (!s || !s->ready) return DSM_ERR_INVALID;
   if (lanes != 0 && lanes != 16 && lanes != 32) return fail(s, DSM_ERR_INVALID, "lanes must be 16 or 32");
   CK(cudaStreamSynchronize(s->st));
+  small_schedule_end(s);
   if (lanes) { s->cfg.lanes = lanes; s->cfg.lock = false; }
   // monodisperse ensembles keep one launch with full-capacity slots unless a
   // smaller slot is asked for (chains that outgrow it finish in the overflow launch)
@@ -858,6 +904,7 @@ extern "C" int dsm_get_class_form(const dsm_sim* s, int32_t* form) {
 extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* best_ms) {
   const dsm::NvtxRange nvtx_range("dsm_autotune");
   if (!s || !s->ready || !(window > 0.0) || s->pending) return DSM_ERR_INVALID;
+  small_schedule_end(s);
   struct Cand { int small, grid, lanes, carve = 0; };
   std::vector<Cand> cands;
   for (int lanes : {32, 16}) {
@@ -1690,7 +1737,8 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   for (int i = 0; i < n; ++i) {
     const bool fl = sims[i]->flow;
     const int co = sims[i]->ck;
-    const int cc = cap_class(sims[i]->cap), cp = co ? sims[i]->cp : 0, ln = sims[i]->cfg.lanes;
+    const int cc = cap_class(sims[i]->cap), cp = co ? sims[i]->cp : 0;
+    const int ln = sims[i]->slot16 > 0 ? 16 : sims[i]->cfg.lanes;
     const bool lk = sims[i]->cfg.lock;
     Group* g = nullptr;
     for (auto& x : groups)
@@ -1765,15 +1813,28 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       for (int q = 0; q < k && all_small; ++q) {
         const dsm_sim* x = sims[g.idx[q]];
         // the small class is the last of an ensemble's classes
-        all_small = !x->classes.empty() && x->classes.back().cfg.lanes == g.lanes;
-        if (all_small) small = std::min(small, x->classes.back().cfg.slot_cap);
+        const int slot16 = x->slot16;
+        all_small = slot16 > 0 ? slot16 < x->cap : !x->classes.empty() && x->classes.back().cfg.lanes == g.lanes;
+        if (all_small) small = std::min(small, slot16 > 0 ? slot16 : x->classes.back().cfg.slot_cap);
       }
-      const bool overflow = all_small && small < cfg.slot_cap;
       LaunchCfg run = cfg;
-      if (overflow) run.slot_cap = small;
-      const int lock_bps = plan_lock(sims[g.idx[0]], run, pre[k]);
-      if (lock_bps == 0) fit_block(g.flow, run, optin);
-      int bps = step_max_blocks_per_sm(g.flow, g.corr, run);
+      // one chain per warp while the chains of all ensembles are resident (small_schedule)
+      int bps = 0, lock_bps = 0;
+      bool one = true;
+      for (int q = 0; q < k && one; ++q) one = sims[g.idx[q]]->slot16 > 0;
+      if (one) {
+        LaunchCfg c;
+        bps = one_per_warp(g.flow, g.corr, cfg.slot_cap, cfg.pmax, optin, c);
+        one = pre[k] <= (long long)bps * s->sm_count * step_tiles(g.flow, c);
+        if (one) run = c;
+      }
+      const bool overflow = !one && all_small && small < cfg.slot_cap;
+      if (!one) {
+        if (overflow) run.slot_cap = small;
+        lock_bps = plan_lock(sims[g.idx[0]], run, pre[k]);
+        if (lock_bps == 0) fit_block(g.flow, run, optin);
+        bps = step_max_blocks_per_sm(g.flow, g.corr, run);
+      }
       if (bps < 1) return fail(s, DSM_ERR_INVALID, "batch slot does not fit shared memory");
       if (lock_bps > 0) bps = std::min(bps, lock_bps);
       const int tiles = step_tiles(g.flow, run);

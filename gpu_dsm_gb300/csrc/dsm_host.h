@@ -139,6 +139,10 @@ struct dsm_sim {
   dsm::StepList carve_list;
   int carve_grid = 0;
   size_t carve_smem = 0;
+  bool shared = false;
+  // one chain per warp because all chains are resident so (small_schedule): the
+  // slot of the two-per-warp plan, which a batch of such ensembles may need; else 0
+  int slot16 = 0;
   // time slices of a launch (EnsDev::subs): the most that pay for this plan, and
   // their per-chain words
   int sub_max = 1;
@@ -159,6 +163,8 @@ struct dsm_sim {
 
 namespace dsm {
 int sim_setup(dsm_sim* s);
+// dsm_create; shared: the ensemble will run next to others on the device
+int sim_create(const dsm_params* p, bool shared, dsm_sim** out);
 // Size-class plan of a polydisperse ensemble; small_cap / big_grid / lanes
 // <= 0 pick the defaults (full-occupancy small slot, large-class grid by work share)
 int plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float margin_sd);

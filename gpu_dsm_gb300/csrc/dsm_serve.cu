@@ -168,7 +168,7 @@ void dsm_server::load_loop() {
     // gets SMs as soon as running blocks retire, not after whole chunks
     dsm_params P = r->P;
     P.stream_priority = prio_greatest;
-    int rc = dsm_create(&P, &sim);
+    int rc = dsm::sim_create(&P, true, &sim);
     if (rc == DSM_OK) rc = dsm_init_equilibrium(sim);
     if (rc == DSM_OK) {
       int32_t grid = 0, bps = 0;
