@@ -1526,32 +1526,49 @@ __global__ void k_gt_reduce(const EnsDev* __restrict__ ensp, double* gsum, long 
 }
 
 // Ensemble average of the window-end stress over non-stalled, non-NaN chains
-// (ensemble_call_block.cu:471-491), FP64, fixed tree order.  out[0..7] sums,
-// out[8] chain count.
-// per_chain: n_chains x 8 floats (NULL: the flow kernel's E.out_stress)
-__global__ void k_stress_reduce(const EnsDev* __restrict__ ensp, const float* __restrict__ per_chain, double* out) {
-  const EnsDev& E = *ensp;
-  __shared__ double red[9][256];
-  double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  const float* src = per_chain != nullptr ? per_chain : E.out_stress;
-  for (int c = threadIdx.x; c < E.n_chains; c += blockDim.x) {
-    const float* s = src + (size_t)c * 8;
-    if (E.cs[c].stall != 0 || s[0] != s[0]) continue;
+// (ensemble_call_block.cu:471-491), FP64, fixed order: chain c into partial c mod
+// 256, then a tree.  out[0..7] sums, out[8] chain count.  One block per sum: the
+// conversions and additions, 16 cycles of an SM's FP64 pipe for each warp
+// instruction, and the latency of the rows bound it (32768 chains: 220 us for the
+// nine sums in one block, 20 in nine).
+__device__ __forceinline__ void stress_sum(const float* __restrict__ rows, const ChainState* __restrict__ cs,
+                                           int n_chains, int q, double* out) {
+  constexpr int U = 8;  // rows in flight per thread
+  __shared__ double red[256];
+  double a = 0.0;
+  for (int c0 = threadIdx.x; c0 < n_chains; c0 += 256 * U) {
+    float first[U], v[U];
+    int stall[U];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) a[q] += (double)s[q];
-    a[8] += 1.0;
-  }
-#pragma unroll
-  for (int q = 0; q < 9; ++q) red[q][threadIdx.x] = a[q];
-  __syncthreads();
-  for (int o = blockDim.x >> 1; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-#pragma unroll
-      for (int q = 0; q < 9; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
+    for (int u = 0; u < U; ++u) {
+      const int c = min(c0 + 256 * u, n_chains - 1);
+      first[u] = rows[(size_t)c * 8];
+      v[u] = q < 8 ? rows[(size_t)c * 8 + q] : 1.0f;
+      stall[u] = cs != nullptr ? cs[c].stall : 0;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + 256 * u < n_chains && stall[u] == 0 && first[u] == first[u]) a += (double)v[u];
+  }
+  red[threadIdx.x] = a;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x < 9) out[threadIdx.x] = red[threadIdx.x][0];
+  if (threadIdx.x == 0) out[q] = red[0];
+}
+// per_chain: n_chains x 8 floats (NULL: the flow kernel's E.out_stress)
+__global__ void __launch_bounds__(256) k_stress_reduce(const EnsDev* __restrict__ ensp,
+                                                       const float* __restrict__ per_chain, double* out) {
+  const EnsDev& E = *ensp;
+  stress_sum(per_chain != nullptr ? per_chain : E.out_stress, E.cs, E.n_chains, blockIdx.x, out);
+}
+// Window blockIdx.y of a flow series
+__global__ void __launch_bounds__(256) k_series_reduce(const EnsDev* __restrict__ ensp, double* out) {
+  const EnsDev& E = *ensp;
+  const size_t w = blockIdx.y;
+  stress_sum(E.win_stress + w * E.n_chains * 8, nullptr, E.n_chains, blockIdx.x, out + w * 9);
 }
 
 // Slots beyond a chain's strands are not maintained by the step kernel; the
@@ -1611,33 +1628,6 @@ __global__ void k_series_begin(EnsDev* ens, const long long* d_win, int stride, 
     ens->n_win = n;
   }
   if (i < n_chains) cs[i].k_next = 0;
-}
-
-// Stress sums of window blockIdx.x of a flow series, in the order of
-// k_stress_reduce (same per-thread strides, same tree)
-__global__ void k_series_reduce(const EnsDev* __restrict__ ensp, double* out) {
-  const EnsDev& E = *ensp;
-  __shared__ double red[9][256];
-  double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  const float* base = E.win_stress + (size_t)blockIdx.x * E.n_chains * 8;
-  for (int c = threadIdx.x; c < E.n_chains; c += blockDim.x) {
-    const float* s = base + (size_t)c * 8;
-    if (s[0] != s[0]) continue;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) a[q] += (double)s[q];
-    a[8] += 1.0;
-  }
-#pragma unroll
-  for (int q = 0; q < 9; ++q) red[q][threadIdx.x] = a[q];
-  __syncthreads();
-  for (int o = blockDim.x >> 1; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-#pragma unroll
-      for (int q = 0; q < 9; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < 9) out[(size_t)blockIdx.x * 9 + threadIdx.x] = red[threadIdx.x][0];
 }
 
 // Window w of a captured series: end time d_win[w] and event cap d_win[n+w]
@@ -1851,17 +1841,17 @@ cudaError_t launch_series_begin(EnsDev* d_ens, const long long* d_win, int strid
   return cudaGetLastError();
 }
 cudaError_t launch_series_reduce(const EnsDev* d_ens, double* out, int n, cudaStream_t st) {
-  k_series_reduce<<<n, 256, 0, st>>>(d_ens, out);
+  k_series_reduce<<<dim3(9, n), 256, 0, st>>>(d_ens, out);
   return cudaGetLastError();
 }
 cudaError_t launch_stress_reduce_dev(const EnsDev* d_ens, double* d_out9, cudaStream_t st) {
-  k_stress_reduce<<<1, 256, 0, st>>>(d_ens, nullptr, d_out9);
+  k_stress_reduce<<<9, 256, 0, st>>>(d_ens, nullptr, d_out9);
   return cudaGetLastError();
 }
 cudaError_t launch_state_stress(const EnsDev* d_ens, int n_chains, float* d_out8, double* d_out9, cudaStream_t st) {
   const long long threads = 32LL * n_chains;
   k_state_stress<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_ens, d_out8);
-  k_stress_reduce<<<1, 256, 0, st>>>(d_ens, d_out8, d_out9);
+  k_stress_reduce<<<9, 256, 0, st>>>(d_ens, d_out8, d_out9);
   return cudaGetLastError();
 }
 
