@@ -143,15 +143,17 @@ __device__ __forceinline__ float shift_minus(const EnsDev& E, int N1, float q1, 
 // One of the two shift components, chosen per lane without divergence:
 // minus = false gives shift_plus, minus = true shift_minus, with the same
 // operations in the same order on selected operands (one exponential per lane).
+// *ok: the exponent is below kExpMost (else the result is not used).
 __device__ __forceinline__ float shift_comp(const EnsDev& E, bool minus, int N1, float q1, int N2, float q2,
-                                            const float4& a, const float4& b) {
+                                            const float4& a, const float4& b, bool* ok) {
   const bool z1 = (q1 == 0.0f), z2 = (q2 == 0.0f);
   const int i = (z1 ? 4 * N1 + (minus ? -1 : 1) : 2 * N1) + (z2 ? 4 * N2 + (minus ? 1 : -1) : 2 * N2);
   const float u = minus ? q2 : q1, ux = minus ? b.x : a.x;
   const float v = minus ? q1 : q2, vy = minus ? a.y : b.y;
   const float arg = __fmaf_rn(u, ux, -__fmul_rn(v, vy));
   const float pw = __fmul_rn(z1 ? 1.0f : (minus ? a.w : a.z), z2 ? 1.0f : (minus ? b.z : b.w));
-  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), m_exp(arg));
+  *ok = arg < kExpMost;
+  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), m_exp_lt88(arg));
   return ((minus ? N1 : N2) > 1) ? w : 0.0f;
 }
 

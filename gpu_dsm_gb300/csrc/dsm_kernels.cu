@@ -315,19 +315,20 @@ __device__ __forceinline__ int update_pairs(const EnsDev& E, Slot& sl, int Z, in
   const int p = p0 + (lane >> 2);
   const bool act = (lane < 4 * cnt) && p >= 0 && p < Z - 1;
   float o = 0.0f;
+  bool ok = true;
   if (act) {
     const int N1 = sl.N[p];
     const int N2 = sl.N[p + 1];
     const float q1 = sl.Q[p].w, q2 = sl.Q[p + 1].w;
     const float4 a = __ldg(&E.NT[N1]), b = __ldg(&E.NT[N2]);
-    const float w = shift_comp(E, k == 2, N1, q1, N2, q2, a, b);
+    const float w = shift_comp(E, k == 2, N1, q1, N2, q2, a, b, &ok);
     // the CD components, loaded by the whole group (same addresses) and selected
     const float tp = sl.T[p], ne = __ldg(&E.NE[N1]).w;
     const float cd = (k == 0) ? tp : ne;
     o = (k == 1 || k == 2) ? w : (E.cd_flag ? cd : 0.0f);
   }
   const float y = __fmul_rn(o, pow2f(S));
-  const bool bad = !(y < 281474976710656.0f);  // 2^(LIMIT_E+1); NaN too
+  const bool bad = !(ok && y < 281474976710656.0f);  // 2^(LIMIT_E+1); NaN too
   const unsigned long long v = f2u64_rn(y);
   unsigned long long tot = v + t.shfl_xor(v, 1);
   tot += t.shfl_xor(tot, 2);

@@ -600,11 +600,12 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
     const int pc = act ? p : 0;
     const int4 c1 = sl.C[pc], c2 = sl.C[pc + 1];
     const int N1 = act ? strand_n(c1.w) : 1, N2 = act ? strand_n(c2.w) : 1;
+    bool ok;
     const float w = shift_comp(E, k == 2, N1, __int_as_float(c1.y), N2, __int_as_float(c2.y), __ldg(&E.NT[N1]),
-                               __ldg(&E.NT[N2]));
+                               __ldg(&E.NT[N2]), &ok);
     const float cde = k == 0 ? __int_as_float(c1.z) : __fmul_rn(E.prefact, (float)(N1 - 1));
     const float y = __fmul_rn((k == 1 || k == 2) ? w : (cd ? cde : 0.0f), sf);
-    *full = __any_sync(FULL_MASK, act && !(y < 281474976710656.0f));  // 2^(LIMIT_E+1); NaN too
+    *full = __any_sync(FULL_MASK, act && !(ok && y < 281474976710656.0f));  // 2^(LIMIT_E+1); NaN too
     const unsigned long long v = f2u64_rn(y);
     unsigned long long tot = v + __shfl_xor_sync(FULL_MASK, v, 1);
     tot += __shfl_xor_sync(FULL_MASK, tot, 2);
@@ -1110,6 +1111,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     const int N2 = act ? strand_n(W2) : 1;
     const float q1 = __int_as_float(ca.y), q2 = __int_as_float(cb.y);
     float wp, wm;
+    bool ok;
     {
       const float4 ta = __ldg(&tNT[N1]), tb = __ldg(&tNT[N2]);
       const bool z1 = (q1 == 0.0f), z2 = (q2 == 0.0f);
@@ -1118,8 +1120,9 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
       const float fp = __ldg(&tFR[i]), fm = __ldg(&tFR[k]);
       const float ep = __fmaf_rn(q1, ta.x, -__fmul_rn(q2, tb.y)), em = __fmaf_rn(q2, tb.x, -__fmul_rn(q1, ta.y));
       const float pp = __fmul_rn(z1 ? 1.0f : ta.z, z2 ? 1.0f : tb.w), pm = __fmul_rn(z1 ? 1.0f : ta.w, z2 ? 1.0f : tb.z);
-      wp = __fmul_rn(__fmul_rn(fp, pp), m_exp(ep));
-      wm = __fmul_rn(__fmul_rn(fm, pm), m_exp(em));
+      ok = ep < kExpMost && em < kExpMost;
+      wp = __fmul_rn(__fmul_rn(fp, pp), m_exp_lt88(ep));
+      wm = __fmul_rn(__fmul_rn(fm, pm), m_exp_lt88(em));
       wp = N2 > 1 ? wp : 0.0f;
       wm = N1 > 1 ? wm : 0.0f;
     }
@@ -1127,7 +1130,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     const float ye = __fmul_rn(__fmul_rn(pfx, (float)(N1 - 1)), sf);
     constexpr float kMost = 281474976710656.0f;  // 2^(LIMIT_E+1); NaN fails the comparisons too
     // (a sum above the limit of one asks for a full pass that changes nothing)
-    const bool bad = act && !(__fadd_rn(__fadd_rn(yp, ym), __fadd_rn(yt, ye)) < kMost);
+    const bool bad = act && !(ok && __fadd_rn(__fadd_rn(yp, ym), __fadd_rn(yt, ye)) < kMost);
     const unsigned long long pt = f2u64_rn(yp) + f2u64_rn(ym) + vt + f2u64_rn(ye);
     const unsigned long long dl = act ? pt - rold : 0ull;
     if (act) {

@@ -68,6 +68,32 @@ __device__ __forceinline__ float m_exp(float x) {
   return (x != x) ? x : res;
 }
 
+// m_exp for x < 88, ten instructions less: the power of two is added to the
+// polynomial's bits (its exponent stays below 255) instead of two products, and a
+// NaN need not pass; the callers take the full rate pass for other x.  The result
+// is m_exp's bit for bit down to -87.3365; below both are 2^-126 within three parts
+// in 10^6, which no fixed-point scale of a rate (at most 2^48 over the largest
+// rate) tells from zero.  (4096 chains of N_K = 463, G(t), 50 tau: 11.71 -> 11.50 ms;
+// MSD of 8192 chains of N_K = 100 6.26 -> 6.23.)
+constexpr float kExpMost = 88.0f;
+__device__ __forceinline__ float m_exp_lt88(float x) {
+  const float xc = fmaxf(x, -87.3365448f);
+  const float MAGIC = 12582912.0f;  // its bits shifted up by 23 are zero
+  const float t = __fmaf_rn(xc, 1.44269504088896341f, MAGIC);
+  const float kf = __fsub_rn(t, MAGIC);
+  float r = __fmaf_rn(kf, -0.693145751953125f, xc);
+  r = __fmaf_rn(kf, -1.428606765330187e-06f, r);
+  float p = 1.98412698e-4f;
+  p = __fmaf_rn(p, r, 1.38888889e-3f);
+  p = __fmaf_rn(p, r, 8.33333333e-3f);
+  p = __fmaf_rn(p, r, 4.16666667e-2f);
+  p = __fmaf_rn(p, r, 1.66666667e-1f);
+  p = __fmaf_rn(p, r, 0.5f);
+  p = __fmaf_rn(p, r, 1.0f);
+  p = __fmaf_rn(p, r, 1.0f);
+  return __int_as_float(__float_as_int(p) + (int)((unsigned)__float_as_int(t) << 23));
+}
+
 __device__ __forceinline__ float m_log(float x) {
   uint32_t b = __float_as_uint(x);
   int e = 0;

@@ -144,3 +144,26 @@ def test_lockstep_abort_between_slices(dsm_mod):
     assert np.array_equal(ca, cb)
     assert np.abs(ga - gb).max() <= 2.0**-22 * np.abs(gb).max()
     assert_bitexact(gpu_state(a), gpu_state(b), what="abort between slices")
+
+
+@pytest.mark.parametrize("n,lanes", [(N, 0), (64, 16), (64, 32)])
+@pytest.mark.parametrize("q", [12.0, 15.0, 17.0, 40.0])
+def test_exponents_beyond_the_short_form(dsm_mod, oracle_mod, n, lanes, q):
+    """Strands so long that sliding exponents reach 54, 84, 108 and 600 (single
+    Kuhn steps): below, near and above the limit of the short exponential, where the
+    full rate pass takes over, with scales far below the start's."""
+    kw = dict(nk=140, n_chains=n, seed=77, beta=0.5)
+    g, o = dsm_mod.Ensemble(lanes_per_chain=lanes, **kw), oracle_mod.Oracle(**kw)
+    g.init_equilibrium()
+    heads, qn, tau = g.get_chains()
+    rng = np.random.default_rng(5)
+    for c in rng.choice(n, n // 4, replace=False):
+        Z = int(heads["Z"][c])
+        if Z > 6:
+            s = int(rng.integers(2, Z - 2))
+            qn[c, s, :3] = np.float32(q) * np.array([0.6, 0.0, 0.8], np.float32)
+    g.set_chains(heads, qn, tau)
+    o.set_state(heads["Z"], qn, tau, T=g.get_ext()["T"])
+    for t in (0.05, 0.5):
+        assert g.advance(t) == o.run(t)
+    assert_bitexact(gpu_state(g), o.get_state(), what=f"|Q|={q}")
