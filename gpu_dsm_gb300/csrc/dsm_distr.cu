@@ -4,6 +4,7 @@
 // shared-memory counters, then one global add per bin), and the lengths |Q| of
 // the internal strands sorted on the device (CUB radix sort) for the Q
 // distribution.
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -46,31 +47,59 @@ __global__ void k_hist_zn(const EnsDev* __restrict__ ensp, unsigned long long* h
 }
 
 // Where each chain's |Q| go in the pooled list, off[n_chains] their number: an
-// exclusive sum of max(Z - 2, 0), one block, each thread a run of chains (32768
-// chains: 10 us, against 2 x 160 for the chains' state on the host and back)
-__global__ void __launch_bounds__(1024) k_qoff(const EnsDev* __restrict__ ensp, long long* off) {
-  const EnsDev& E = *ensp;
-  __shared__ long long part[32];
-  const int n = E.n_chains, per = (n + 1023) / 1024, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long c0 = (long long)threadIdx.x * per, c1 = min(c0 + per, (long long)n);
-  long long sum = 0;
-#pragma unroll 8
-  for (long long c = c0; c < c1; ++c) sum += max(E.cs[c].Z - 2, 0);
-  long long v = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long u = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += u;
-  }
-  if (lane == 31) part[warp] = v;
+// exclusive sum of max(Z - 2, 0).  Each block a run of `per` chains, its total first
+// (k_qsum), then the offsets behind the totals of the blocks before it (k_qoff).
+// (32768 chains: 9 us, 60 in one block, whose reads of the chains' state, 80 bytes
+// apart, bound it; against 160 for the state on the host and the offsets back.)
+__device__ __forceinline__ long long block_sum(long long v, long long* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  long long before = v - sum;
-  for (int w = 0; w < warp; ++w) before += part[w];
-#pragma unroll 8
-  for (long long c = c0; c < c1; ++c) {
-    off[c] = before;
-    before += max(E.cs[c].Z - 2, 0);
+  long long t = 0;
+  for (int w = 0; w < 8; ++w) t += red[w];
+  __syncthreads();
+  return t;
+}
+__global__ void __launch_bounds__(256) k_qsum(const EnsDev* __restrict__ ensp, int per, long long* part) {
+  __shared__ long long red[8];
+  const EnsDev& E = *ensp;
+  const long long c0 = (long long)blockIdx.x * per, c1 = min(c0 + per, (long long)E.n_chains);
+  long long v = 0;
+  for (long long c = c0 + threadIdx.x; c < c1; c += 256) v += max(E.cs[c].Z - 2, 0);
+  const long long t = block_sum(v, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
+}
+__global__ void __launch_bounds__(256) k_qoff(const EnsDev* __restrict__ ensp, int per,
+                                              const long long* __restrict__ part, long long* off) {
+  __shared__ long long red[8];
+  const EnsDev& E = *ensp;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long c0 = (long long)blockIdx.x * per, c1 = min(c0 + per, (long long)E.n_chains);
+  long long v = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += 256) v += part[b];
+  long long base = block_sum(v, red);
+  for (long long r = c0; r < c1; r += 256) {
+    const long long c = r + threadIdx.x;
+    const long long z = c < c1 ? max(E.cs[c].Z - 2, 0) : 0;
+    long long inc = z;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) red[warp] = inc;
+    __syncthreads();
+    long long before = base, all = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += red[w];
+      all += red[w];
+    }
+    if (c < c1) off[c] = before + inc - z;
+    base += all;
+    __syncthreads();
   }
-  if (threadIdx.x == 1023) off[n] = before;
+  if (c1 == (long long)E.n_chains && c0 < c1 && threadIdx.x == 0) off[c1] = base;
 }
 
 // |Q| of the internal strands 1..Z-2 of chain c at out[off[c] ..]
@@ -124,10 +153,12 @@ extern "C" int dsm_zn_hist(dsm_sim* s, uint64_t* z_counts, int32_t z_bins, uint6
 extern "C" int dsm_q_sorted(dsm_sim* s, float* q, int64_t* n) {
   if (!s || !s->ready || !n) return DSM_ERR_INVALID;
   const int nc = s->P.n_chains;
-  long long* d_off = nullptr;
+  long long* d_off = nullptr;  // [nc + 1] offsets, then the blocks' totals
   long long tot = 0;
-  CKD(cudaMallocAsync((void**)&d_off, (size_t)(nc + 1) * sizeof(long long), s->st));
-  k_qoff<<<1, 1024, 0, s->st>>>(s->d_ens, d_off);
+  const int per = std::max(256, (nc + s->sm_count - 1) / s->sm_count), blocks = (nc + per - 1) / per;
+  CKD(cudaMallocAsync((void**)&d_off, (size_t)(nc + 1 + blocks) * sizeof(long long), s->st));
+  k_qsum<<<blocks, 256, 0, s->st>>>(s->d_ens, per, d_off + nc + 1);
+  k_qoff<<<blocks, 256, 0, s->st>>>(s->d_ens, per, d_off + nc + 1, d_off);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&tot, d_off + nc, sizeof(tot), cudaMemcpyDeviceToHost, s->st);

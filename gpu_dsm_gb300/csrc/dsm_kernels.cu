@@ -1531,7 +1531,7 @@ __global__ void k_gt_reduce(const EnsDev* __restrict__ ensp, double* gsum, long 
 // 256, then a tree.  out[0..7] sums, out[8] chain count.  One block per sum: the
 // conversions and additions, 16 cycles of an SM's FP64 pipe for each warp
 // instruction, and the latency of the rows bound it (32768 chains: 220 us for the
-// nine sums in one block, 20 in nine).
+// nine sums in one block, 37 in nine).
 __device__ __forceinline__ void stress_sum(const float* __restrict__ rows, const ChainState* __restrict__ cs,
                                            int n_chains, int q, double* out) {
   constexpr int U = 8;  // rows in flight per thread

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 KAP = (0.0, 2.0e-3, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0)
 
 
-@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1023, 1025, 2047, 2049, 5000])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1023, 1025, 2049, 5000, 39000])
 def test_sums_and_lists(dsm_mod, n):
     e = dsm_mod.Ensemble(nk=30, n_chains=n, seed=95)
     e.init_equilibrium()
