@@ -215,11 +215,12 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_
 //     G(t)    N_K 150 2.00e9 / 2.17e9   N_K 200 1.95e9 / 1.89e9   N_K 463 1.96e9 / 1.04e9
 //   beta 2    N_K 100 3.35e9 / 2.84e9   N_K 300 3.20e9 / 2.33e9
 //     G(t)    N_K 100 2.01e9 / 2.56e9   N_K 150 2.52e9 / 2.60e9   N_K 200 3.01e9 / 2.29e9
-// (default_schedule adds: more chains than the tiles hold at once.)  Strand
+// (default_schedule adds: more chains than the tiles hold at once.)  Not in the
+// server, whose memory budget does not count the kernel's buffers.  Strand
 // sizes and the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
 static bool prefer_lock(const dsm_sim* s) {
   const dsm_params& P = s->P;
-  if (P.lanes_per_chain != 0 || s->flow || s->poly || s->nkmax >= 16384) return false;
+  if (P.lanes_per_chain != 0 || s->flow || s->poly || s->shared || !s->lock_fits || s->nkmax >= 16384) return false;
   const double f = (2.0 + 1.0 / (double)P.beta) / 3.0;
   return (double)P.nk >= (s->corr ? 150.0 * std::max(1.0, f) : 100.0 * f);
 }
@@ -293,12 +294,13 @@ int dsm::sim_setup(dsm_sim* s) {
   const size_t n = (size_t)P.n_chains, cap = (size_t)s->cap;
   size_t need = n * cap * (16 + 4) + n * sizeof(ChainState) + n * 8 * 4;
   if (s->corr) need += n * s->levels * ((size_t)s->cp * (12 + 8) + 12 + 16);
-  const size_t kahan_bytes = s->corr && prefer_lock(s) ? n * ((size_t)s->cp * sizeof(float2) + 3 * kCorrBuf * sizeof(float)) : 0;
-  need += kahan_bytes;
   size_t fre = 0, tot = 0;
   CK(cudaMemGetInfo(&fre, &tot));
   if (need + (64ull << 20) > fre) return fail(s, DSM_ERR_MEMORY, "ensemble needs " + std::to_string(need >> 20) + " MiB of device memory, " + std::to_string(fre >> 20) + " MiB free");
   s->bytes = need;
+  // what the lockstep kernel needs besides (plan_buffers); without room, tiles
+  const size_t more = n * (sizeof(Slice) + (s->corr ? (size_t)s->cp * sizeof(float2) + 3 * kCorrBuf * sizeof(float) : 0));
+  s->lock_fits = need + more + (64ull << 20) <= fre;
 
   // tables
   std::vector<float> tb;

@@ -139,7 +139,8 @@ struct dsm_sim {
   dsm::StepList carve_list;
   int carve_grid = 0;
   size_t carve_smem = 0;
-  bool shared = false;
+  bool shared = false;     // runs next to other ensembles on the device (dsm_server)
+  bool lock_fits = false;  // device memory for the lockstep kernel's buffers
   // one chain per warp because all chains are resident so (small_schedule): the
   // slot of the two-per-warp plan, which a batch of such ensembles may need; else 0
   int slot16 = 0;

@@ -8,8 +8,9 @@ the step kernel's event loop reads the SM clock at each phase boundary and
 sums the cycles per phase over chains) and runs the equilibrium melt of the
 headline workload's parameters (N_K = 200, beta = 1, G(t) with p = 64, m = 8):
 
-  load    16384 chains, the library's default schedule (32 chain tiles per
-          SM), one 5 tau_K window after three warm-up windows
+  load    16384 chains in the tile kernel (the default there is the lockstep
+          kernel, which has no phase clocks), 143-strand slots, 32 chain
+          tiles per SM, one 5 tau_K window after three warm-up windows
   warp    304 chains, one warp (two 16-lane tiles) per SM, 200 tau_K
   single  one chain on the whole GPU (16 and 32 lanes), 5000 tau_K: the
           latency of a chain that shares nothing
@@ -54,10 +55,12 @@ def _load():
     return api, lib
 
 
-def run_case(api, lib, tag: str, n: int, window: float, warm: int, **kw) -> dict:
+def run_case(api, lib, tag: str, n: int, window: float, warm: int, small_slot: int = 0, **kw) -> dict:
     e = api.Ensemble(beta=1.0, nk=200, n_chains=n, eq_type=1, sync_dt=1.0, t_end=1.0e7, seed=1, corr_p=64, corr_m=8,
                      **kw)
     try:
+        if small_slot:
+            e.set_schedule(small_slot=small_slot, lanes=16)
         e.init_equilibrium()
         t = 0.0
         for _ in range(warm):
@@ -106,7 +109,7 @@ def main(argv=None) -> int:
     api, lib = _load()
     for c in cases:
         if c == "load":
-            out = [run_case(api, lib, "load", 16384, 5.0, 3)]
+            out = [run_case(api, lib, "load", 16384, 5.0, 3, small_slot=143)]
         elif c == "warp":
             out = [run_case(api, lib, "one_warp_per_sm", 304, 200.0, 1, lanes_per_chain=16, warps_per_block=1)]
         elif c == "single":
