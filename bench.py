@@ -256,8 +256,9 @@ def latency_probe(args, device: int, f_hz: float, tiles_per_sm: int, value: floa
     run as one warp (two 16-lane chain tiles) per block, so that each SM holds
     a single warp; their events per second give the critical-path cycles per
     event of a chain that waits for nothing but its own dependencies.  The
-    bound is every resident chain tile of the headline schedule running at that
-    speed; frac = achieved / bound."""
+    bound is tiles_per_sm tiles of that kernel on every SM running at that
+    speed; frac = achieved / bound.  (The headline ensemble itself runs the
+    lockstep kernel, for which this is a comparison, not a bound.)"""
     import gpu_dsm_gb300 as dsm
 
     n = 2 * 152

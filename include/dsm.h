@@ -73,7 +73,9 @@ typedef struct dsm_params {
   const int32_t* nk_chain; /* per-chain N_K (polydisperse melt) or NULL */
   int32_t warps_per_block; /* step-kernel block size in warps; 0 = autotuned */
   int32_t s0;              /* initial fixed-point scale exponent; 0 = 40 */
-  int32_t lanes_per_chain; /* 32: one chain per warp, 16: two chains per warp; 0 = auto */
+  int32_t lanes_per_chain; /* 32: one chain per warp, 16: two chains per warp; 0 = auto (by the
+                              chains' number and length; large monodisperse equilibrium
+                              ensembles then run in lockstep, dsm_lockstep.cu) */
   int32_t stream_priority; /* CUDA priority of the handle's streams (0 = default; lower
                               values are scheduled first, clamped to the device's range) */
   float gex_a, gex_b;      /* pd_flag = 1: polydisp.dat a, b of the GEX background law */
@@ -206,7 +208,9 @@ int dsm_pcd(double beta, int32_t nk, double* out);
  * small slot.  Results do not depend on the schedule (state, flow stress and
  * G(t) to the bit; the MSD centre-of-mass sums to rounding).  Arguments <= 0 choose
  * the defaults (largest slot with 4 blocks per SM; large-class blocks in
- * proportion to its share of the work; lanes of the handle; 5 sd).  No
+ * proportion to its share of the work; lanes of the handle; 5 sd).  Explicit
+ * lanes run the tile kernel; a lockstep plan keeps its kernel otherwise and
+ * reports the tiles' lanes.  No
  * counterpart in the reference (one thread per chain, ensemble_kernel.cu). */
 int dsm_set_schedule(dsm_sim* sim, int32_t small_slot, int32_t large_grid, int32_t lanes, float z_margin_sd);
 /* Current schedule: n_classes (0 = one launch over all chains), then per
