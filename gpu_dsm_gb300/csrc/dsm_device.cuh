@@ -25,10 +25,11 @@ __device__ __forceinline__ unsigned long long quant(float x, float sf) {
 // cycles of latency and as many cycles of pipe occupancy per warp instruction
 // (about 31 cycles of latency for this form).  update_pairs converts the
 // components of every recomputed pair on the critical path of each event.
-// Where one or two conversions stand alone (event classification, dt), or in
-// the flow pass that converts every pair of the chain each event, the extra
-// instructions of this form cost more than they save at full occupancy, and
-// the instruction stays (each measured on the N_K = 200 melt and shear).
+// Where one or two conversions stand alone (event classification, dt) the extra
+// instructions of this form cost more than they save at full occupancy, and the
+// instruction stays; the flow pass, which converts every pair of the chain each
+// event, takes this form for two of a pair's four components (each measured on the
+// N_K = 200 melt and shear).
 //
 // f2u64_rn: y in [0, 2^63) (or -0.0), the value llrint(y) takes.  Below 2^23
 // adding 2^23 rounds y to an integer (the sum's ulp is 1) and the sum's bit
@@ -119,24 +120,29 @@ __device__ __forceinline__ PcdDev partner_pcd(const EnsDev& E, uint32_t w, bool 
 // Shift components of the pair (strand j, strand j+1), ensemble_kernel.cu:149-179:
 // wp moves a Kuhn step from strand j+1 into strand j, wm the reverse.
 // a = NT[N1], b = NT[N2].
+// SHORT: by m_exp_lt88, *ok cleared when the exponent is out of its range.
+template <bool SHORT>
 __device__ __forceinline__ float shift_plus(const EnsDev& E, int N1, float q1, int N2, float q2, const float4& a,
-                                            const float4& b) {
+                                            const float4& b, bool* ok = nullptr) {
   const bool z1 = (q1 == 0.0f), z2 = (q2 == 0.0f);
   const int i = (z1 ? 4 * N1 + 1 : 2 * N1) + (z2 ? 4 * N2 - 1 : 2 * N2);
   const float t2 = __fmul_rn(q2, b.y);
   const float arg = __fmaf_rn(q1, a.x, -t2);
   const float pw = __fmul_rn(z1 ? 1.0f : a.z, z2 ? 1.0f : b.w);
-  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), m_exp(arg));
+  if (SHORT) *ok = *ok && arg < kExpMost;
+  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), SHORT ? m_exp_lt88(arg) : m_exp(arg));
   return (N2 > 1) ? w : 0.0f;
 }
+template <bool SHORT>
 __device__ __forceinline__ float shift_minus(const EnsDev& E, int N1, float q1, int N2, float q2, const float4& a,
-                                             const float4& b) {
+                                             const float4& b, bool* ok = nullptr) {
   const bool z1 = (q1 == 0.0f), z2 = (q2 == 0.0f);
   const int i = (z1 ? 4 * N1 - 1 : 2 * N1) + (z2 ? 4 * N2 + 1 : 2 * N2);
   const float t1 = __fmul_rn(q1, a.y);
   const float arg = __fmaf_rn(q2, b.x, -t1);
   const float pw = __fmul_rn(z1 ? 1.0f : a.w, z2 ? 1.0f : b.z);
-  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), m_exp(arg));
+  if (SHORT) *ok = *ok && arg < kExpMost;
+  const float w = __fmul_rn(__fmul_rn(__ldg(&E.FRIC[i]), pw), SHORT ? m_exp_lt88(arg) : m_exp(arg));
   return (N1 > 1) ? w : 0.0f;
 }
 

@@ -271,15 +271,19 @@ __device__ __forceinline__ void move_strands(Slot& sl, int lo, int Z, int dir, c
 }
 
 // float components {CD destruction, shift +1, shift -1, CD creation} of pair p
-// (ensemble_kernel.cu:149-181,304-414)
-__device__ __forceinline__ void pair_floats(const EnsDev& E, const Slot& sl, int p, float o[4]) {
+// (ensemble_kernel.cu:149-181,304-414); SHORT: by the short exponential, false when
+// an exponent is out of its range
+template <bool SHORT>
+__device__ __forceinline__ bool pair_floats(const EnsDev& E, const Slot& sl, int p, float o[4]) {
   const int N1 = sl.N[p], N2 = sl.N[p + 1];
   const float q1 = sl.Q[p].w, q2 = sl.Q[p + 1].w;
   const float4 a = __ldg(&E.NT[N1]), b = __ldg(&E.NT[N2]);
   o[0] = E.cd_flag ? sl.T[p] : 0.0f;
-  o[1] = shift_plus(E, N1, q1, N2, q2, a, b);
-  o[2] = shift_minus(E, N1, q1, N2, q2, a, b);
+  bool ok = true;
+  o[1] = shift_plus<SHORT>(E, N1, q1, N2, q2, a, b, &ok);
+  o[2] = shift_minus<SHORT>(E, N1, q1, N2, q2, a, b, &ok);
   o[3] = E.cd_flag ? __ldg(&E.NE[N1]).w : 0.0f;
+  return ok;
 }
 
 // Chain-end component q (0 CD creation at the tail, 1 SD creation head, 2 SD
@@ -347,6 +351,16 @@ __device__ __forceinline__ int update_pairs(const EnsDev& E, Slot& sl, int Z, in
 // track the max exponent; apply the scale rule shared with the oracle (lower on
 // overflow; flow raises again once 2^16 of headroom is free) and requantise if S
 // changes.  Returns the new S; *flags_out gets NaN/inf bits (S kept then).
+//
+// Flow runs it every event: issue slots (66 % busy) and the FP64 pipe's conversions
+// (72 %) bound it together.  So the two sliding components are quantised by 32-bit
+// operations (all four: slower, the instructions cost more than the pipe), one
+// maximum over the components' bits stands for the NaN, infinity and exponent
+// checks, and the exponentials are m_exp_lt88; a lane that meets a component or
+// exponent out of range goes over its pairs again in full.  One vote in place of
+// the two tile reductions below is slower, 9 % at N_K = 30.  Shear, Wi 10, N_K = 100
+// 7.07 -> 6.63 ms (16384 chains, 25 tau), N_K = 200 11.9 -> 10.6 (15 tau), N_K = 30
+// 4.2 -> 3.85 (50 tau), 4096 chains of N_K = 50 2.14 -> 2.07 (50 tau).
 template <bool FLOW, int W>
 __device__ __forceinline__ int full_rates_body(const EnsDev& E, Slot& sl, int Z, int S, float wz1, const Tile<W>& t,
                                                int* flags_out) {
@@ -359,21 +373,45 @@ __device__ __forceinline__ int full_rates_body(const EnsDev& E, Slot& sl, int Z,
   // maximum (any flag keeps the scale), so the largest |bits| gives it, and
   // a NaN is exactly an |bits| above the infinity pattern
   unsigned mx = 0u;
-  for (int p = lane; p < np; p += W) {
-    float o[4];
-    pair_floats(E, sl, p, o);
-    unsigned long long tot = 0;
+  auto in_full = [&]() {
+    for (int p = lane; p < np; p += W) {
+      float o[4];
+      pair_floats<false>(E, sl, p, o);
+      unsigned long long tot = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const unsigned b = __float_as_uint(o[q]);
-      mx = max(mx, b & 0x7fffffffu);
-      if (b == 0x7f800000u) flags |= 2;
-      tot += quant(o[q], sf);
+      for (int q = 0; q < 4; ++q) {
+        const unsigned b = __float_as_uint(o[q]);
+        mx = max(mx, b & 0x7fffffffu);
+        if (b == 0x7f800000u) flags |= 2;
+        tot += quant(o[q], sf);
+      }
+      sl.R[p] = tot;
+      sl.P[p] = quant(o[1], sf);
     }
-    sl.R[p] = tot;
-    sl.P[p] = quant(o[1], sf);
+    if (mx > 0x7f800000u) flags |= 1;
+  };
+  if constexpr (FLOW) {
+    bool ok = true;
+    for (int p = lane; p < np; p += W) {
+      float o[4];
+      ok = pair_floats<true>(E, sl, p, o) && ok;
+      unsigned long long tot = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        mx = max(mx, __float_as_uint(o[q]));
+        const unsigned long long v = (q == 1 || q == 2) ? f2u64_rn(__fmul_rn(o[q], sf)) : quant(o[q], sf);
+        if (q == 1) sl.P[p] = v;
+        tot += v;
+      }
+      sl.R[p] = tot;
+    }
+    if (mx >= 0x7f800000u || !ok) {
+      mx = 0u;
+      in_full();
+    }
+  } else {
+    in_full();
   }
-  if (mx > 0x7f800000u) flags |= 1;
   if (mx >= 0x00800000u) emax = max(emax, (int)(mx >> 23) - 127);
   float ev = 0.0f;
   if (lane < NEND) {
@@ -392,7 +430,7 @@ __device__ __forceinline__ int full_rates_body(const EnsDev& E, Slot& sl, int Z,
     const float sf2 = pow2f(Snew);
     for (int p = lane; p < np; p += W) {
       float o[4];
-      pair_floats(E, sl, p, o);
+      pair_floats<false>(E, sl, p, o);
       const unsigned long long qp = quant(o[1], sf2);
       sl.R[p] = quant(o[0], sf2) + qp + quant(o[2], sf2) + quant(o[3], sf2);
       sl.P[p] = qp;
@@ -1477,8 +1515,8 @@ __global__ void __launch_bounds__(128) k_init(const EnsDev* __restrict__ ensp, i
     const float q1 = gq2[p], q2 = gq2[p + 1];
     const float4 a = __ldg(&E.NT[N1]), b = __ldg(&E.NT[N2]);
     emax = max(emax, fexp(E.cd_flag ? gt[p] : 0.0f));
-    emax = max(emax, fexp(shift_plus(E, N1, q1, N2, q2, a, b)));
-    emax = max(emax, fexp(shift_minus(E, N1, q1, N2, q2, a, b)));
+    emax = max(emax, fexp(shift_plus<false>(E, N1, q1, N2, q2, a, b)));
+    emax = max(emax, fexp(shift_minus<false>(E, N1, q1, N2, q2, a, b)));
     emax = max(emax, fexp(E.cd_flag ? __ldg(&E.NE[N1]).w : 0.0f));
   }
   if (lane < NEND) {

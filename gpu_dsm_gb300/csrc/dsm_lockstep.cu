@@ -141,8 +141,8 @@ __device__ __forceinline__ void lock_pair(const EnsDev& E, const LSlot& sl, int 
   const float q1 = __int_as_float(c1.y), q2 = __int_as_float(c2.y);
   const float4 a = __ldg(&E.NT[N1]), b = __ldg(&E.NT[N2]);
   o[0] = E.cd_flag ? __int_as_float(c1.z) : 0.0f;
-  o[1] = shift_plus(E, N1, q1, N2, q2, a, b);
-  o[2] = shift_minus(E, N1, q1, N2, q2, a, b);
+  o[1] = shift_plus<false>(E, N1, q1, N2, q2, a, b);
+  o[2] = shift_minus<false>(E, N1, q1, N2, q2, a, b);
   o[3] = E.cd_flag ? __ldg(&E.NE[N1]).w : 0.0f;
 }
 
