@@ -276,7 +276,7 @@ def latency_probe(args, device: int, f_hz: float, tiles_per_sm: int, value: floa
             f"{ev} events, {lw['grid']} blocks", "resident_chain_tiles_per_sm": tiles_per_sm,
             "achieved": value / 1e9, "peak": bound / 1e9, "unit": "Gevents/s", "frac": value / bound,
             "cycles_per_event_at_load": 152 * tiles_per_sm * f_hz / value,
-            "note": "peak = 152 SMs x resident chain tiles x clock / critical-path cycles per event"}
+            "note": "peak = 152 SMs x resident chain tiles x clock / critical-path cycles per event of the tile kernel"}
 
 
 def spawn_ranks(args) -> int:
