@@ -1104,7 +1104,16 @@ __global__ void __launch_bounds__(128, MB) k_step(const EnsDev* __restrict__ ens
       j0 = lane * cw;
       const int j1 = min(j0 + cw, ne);
       unsigned long long part = 0;
-      for (int jj = j0; jj < j1; ++jj) part += sl.R[jj];
+      // (equilibrium: not unrolled, four to nine pairs a lane; the code costs more
+      // than the branches, 40 tau of 16384 chains of N_K = 50, p = 16: 3.10 -> 2.90
+      // ms, MSD of 8192 of N_K = 100 5.64 -> 5.20.  Flow does it every event: a
+      // series of 4096 chains of N_K = 50 2.19 unrolled, 2.27 not)
+      if constexpr (FLOW) {
+        for (int jj = j0; jj < j1; ++jj) part += sl.R[jj];
+      } else {
+#pragma unroll 1
+        for (int jj = j0; jj < j1; ++jj) part += sl.R[jj];
+      }
       incl = tile_scan(t, part);
       excl = incl - part;
       tot = t.shfl(incl, W - 1);
