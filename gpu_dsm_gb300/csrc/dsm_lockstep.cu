@@ -961,7 +961,9 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
         continue;
       }
       idle = 0;
+      // what the slide lanes wrote before the request, seen by lane 0, now by all
       __threadfence_block();
+      __syncwarp();
       const LSlot sl = lock_slot(slots + (size_t)b * sbytes, slot_cap, SB);
       const bool done = lock_serve<CK, SUBS, SB>(ens, n_ens, prefix, n_items, subs, work, slot_cap, sl, 1u << b, ctl,
                                                  abort_flag, status, lst);
@@ -1008,6 +1010,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     const bool res = !run && (dn & bit) != 0u;
     if (__any_sync(FULL_MASK, res)) {
       __threadfence_block();
+      __syncwarp();  // (as in the service warps)
       if (res) {
         if (gl == 0) atomicAnd(&ctl->done, ~bit);
         const int what = h->fresh;
@@ -1133,6 +1136,9 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     const bool bad = act && !(ok && __fadd_rn(__fadd_rn(yp, ym), __fadd_rn(yt, ye)) < kMost);
     const unsigned long long pt = f2u64_rn(yp) + f2u64_rn(ym) + vt + f2u64_rn(ye);
     const unsigned long long dl = act ? pt - rold : 0ull;
+    // (shuffles and votes do not order memory: the neighbours' loads of a strand
+    // come before its store, and the chain-end loads below after it)
+    __syncwarp();
     if (act) {
       sl.R[p] = pt;
       sl.C[p].x = __float_as_int(wp);
@@ -1154,6 +1160,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     // a slide next to a chain end changes the chain-end rates
     const bool near = slide && (jj <= 1 || jj + 1 >= Z - 2);
     if (__any_sync(FULL_MASK, near)) {
+      __syncwarp();
       // lane 0 the head, lane 1 the tail (its sliding creation, or with one
       // Kuhn step its sliding destruction), lane 2 the tail's CD creation
       // (ensemble_kernel.cu:219-260; the others of the five rates are zero)
