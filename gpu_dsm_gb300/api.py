@@ -142,6 +142,8 @@ def load_library() -> C.CDLL:
     lib.dsm_set_schedule.restype = C.c_int
     lib.dsm_get_schedule.argtypes = [vp, C.POINTER(i32), vp]
     lib.dsm_get_schedule.restype = C.c_int
+    lib.dsm_set_wait_polls.argtypes = [vp, C.c_uint32]
+    lib.dsm_set_wait_polls.restype = C.c_int
     lib.dsm_set_class_form.argtypes = [vp, i32]
     lib.dsm_set_class_form.restype = C.c_int
     lib.dsm_get_class_form.argtypes = [vp, C.POINTER(i32)]
@@ -452,6 +454,11 @@ class Ensemble:
     def set_schedule(self, small_slot: int = 0, large_grid: int = 0, lanes: int = 0, z_margin_sd: float = 0.0) -> None:
         """Size-class launch schedule of a polydisperse ensemble (dsm_set_schedule)."""
         self._check(self._lib.dsm_set_schedule(self._h, small_slot, large_grid, lanes, z_margin_sd))
+
+    def set_wait_polls(self, polls: int) -> None:
+        """Polls after which a wait between the warps of a launch that makes no progress
+        gives up, 0 for the default (dsm_set_wait_polls)."""
+        self._check(self._lib.dsm_set_wait_polls(self._h, polls))
 
     def set_class_form(self, form: int) -> None:
         """0: size classes as concurrent launches; 1: large, middle and small

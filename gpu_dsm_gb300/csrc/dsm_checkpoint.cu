@@ -117,6 +117,7 @@ int fail(dsm_sim* s, int code, const std::string& m) {
 extern "C" int dsm_checkpoint_save(dsm_sim* s, const char* path) {
   const dsm::NvtxRange nvtx_range("dsm_checkpoint_save");
   if (!s || !s->ready || !path || s->pending) return DSM_ERR_INVALID;
+  if (s->lost) return dsm::state_lost(s);
   const std::vector<Part> ps = parts(s);
   Header h = header_of(s);
   std::vector<std::vector<unsigned char>> host(ps.size());
@@ -186,6 +187,7 @@ extern "C" int dsm_checkpoint_load(dsm_sim* s, const char* path) {
   }
   const cudaError_t e = cudaStreamSynchronize(s->st);
   if (e != cudaSuccess) return fail(s, DSM_ERR_CUDA, std::string("restore copy: ") + cudaGetErrorString(e));
+  s->lost = false;
   s->t_done = h.t_done;
   s->t_window = h.t_done;
   s->events_total = h.events_total;

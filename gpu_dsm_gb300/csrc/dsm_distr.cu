@@ -132,6 +132,7 @@ int fail(dsm_sim* s, int code, const char* msg) {
 
 extern "C" int dsm_zn_hist(dsm_sim* s, uint64_t* z_counts, int32_t z_bins, uint64_t* n_counts, int32_t n_bins) {
   if (!s || !s->ready || z_bins < 1 || n_bins < 1 || !z_counts || !n_counts) return DSM_ERR_INVALID;
+  if (s->lost) return dsm::state_lost(s);
   const size_t shm = (size_t)(z_bins + n_bins) * sizeof(unsigned int);
   if (shm > 200 * 1024) return fail(s, DSM_ERR_INVALID, "histogram ranges too large for shared memory");
   unsigned long long* d = nullptr;
@@ -152,6 +153,7 @@ extern "C" int dsm_zn_hist(dsm_sim* s, uint64_t* z_counts, int32_t z_bins, uint6
 
 extern "C" int dsm_q_sorted(dsm_sim* s, float* q, int64_t* n) {
   if (!s || !s->ready || !n) return DSM_ERR_INVALID;
+  if (s->lost) return dsm::state_lost(s);
   const int nc = s->P.n_chains;
   long long* d_off = nullptr;  // [nc + 1] offsets, then the blocks' totals
   long long tot = 0;

@@ -906,6 +906,7 @@ extern "C" int dsm_get_class_form(const dsm_sim* s, int32_t* form) {
 extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* best_ms) {
   const dsm::NvtxRange nvtx_range("dsm_autotune");
   if (!s || !s->ready || !(window > 0.0) || s->pending) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   small_schedule_end(s);
   struct Cand { int small, grid, lanes, carve = 0; };
   std::vector<Cand> cands;
@@ -975,6 +976,7 @@ extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* bes
 
 extern "C" int dsm_get_r1(dsm_sim* s, float* r1) {
   if (!s || !s->ready || !r1) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   const size_t n = s->P.n_chains;
   std::vector<ChainState> cs(n);
   CK(cudaMemcpyAsync(cs.data(), s->d_cs, n * sizeof(ChainState), cudaMemcpyDeviceToHost, s->st));
@@ -1036,6 +1038,7 @@ extern "C" int dsm_init_equilibrium(dsm_sim* s) {
   if (rc) return rc;
   CK(launch_init(s->d_ens, s->h, s->cap, s->st));
   CK(cudaStreamSynchronize(s->st));
+  s->lost = false;
   return DSM_OK;
 }
 
@@ -1087,12 +1090,14 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
   int rc = reset_corr(s);
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
+  s->lost = false;
   return DSM_OK;
 }
 
 extern "C" int dsm_get_chains(dsm_sim* s, dsm_chain_head* heads, dsm_float4* QN, float* tau) {
   const dsm::NvtxRange nvtx_range("dsm_get_chains");
   if (!s || !s->ready) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   const size_t n = s->P.n_chains, cap = s->cap;
   // slots beyond Z are not maintained on the device: zero them there, so the
   // copies come back in the reference layout without a host pass
@@ -1115,6 +1120,7 @@ extern "C" int dsm_get_chains(dsm_sim* s, dsm_chain_head* heads, dsm_float4* QN,
 extern "C" int dsm_get_ext(dsm_sim* s, int64_t* T, uint64_t* steps, float* dt_prev, int32_t* stall,
                            int32_t* scale, uint64_t* hash) {
   if (!s || !s->ready) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   const size_t n = s->P.n_chains;
   std::vector<ChainState> cs(n);
   CK(cudaMemcpyAsync(cs.data(), s->d_cs, n * sizeof(ChainState), cudaMemcpyDeviceToHost, s->st));
@@ -1133,6 +1139,7 @@ extern "C" int dsm_get_ext(dsm_sim* s, int64_t* T, uint64_t* steps, float* dt_pr
 extern "C" int dsm_set_ext(dsm_sim* s, const int64_t* T, const uint64_t* steps, const float* dt_prev,
                            const int32_t* stall, const int32_t* scale) {
   if (!s || !s->ready) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   const size_t n = s->P.n_chains;
   std::vector<ChainState> cs(n);
   CK(cudaMemcpyAsync(cs.data(), s->d_cs, n * sizeof(ChainState), cudaMemcpyDeviceToHost, s->st));
@@ -1175,6 +1182,7 @@ static int enqueue_classes(dsm_sim* s) {
     l.order = s->d_order + k.first;
     l.defer = s->d_defer;
     l.n_defer = s->d_works + 3;
+    l.polls = s->wait_polls;
     cudaStream_t st = k.stream == 1 ? s->side : k.stream == 2 ? s->side2 : k.stream == 3 ? s->side3 : s->st;
     unsigned int* work = s->d_works + (k.stream == 1 ? 1 : k.stream == 2 ? 4 : k.stream == 3 ? 5 : 0);
     CK(launch_step(s->d_ens, 1, s->d_prefix, k.count, work, s->flow, s->ck, k.cfg, s->d_abort, s->d_status,
@@ -1218,9 +1226,11 @@ static int enqueue_slice_flush(dsm_sim* s) {
 static int enqueue_step(dsm_sim* s) {
   if (s->sub_max > 1) CK(cudaMemsetAsync(s->d_slice, 0, (size_t)s->P.n_chains * sizeof(Slice), s->st));
   if (s->classes.empty()) {
+    StepList l;
+    l.polls = s->wait_polls;
     CK(cudaMemsetAsync(s->d_work, 0, sizeof(unsigned int), s->st));
     CK(launch_step(s->d_ens, 1, s->d_prefix, (long long)s->P.n_chains, s->d_work, s->flow, s->ck, s->cfg,
-                   s->d_abort, s->d_status, s->grid, s->st));
+                   s->d_abort, s->d_status, s->grid, s->st, l));
     return enqueue_slice_flush(s);
   }
   CK(cudaMemsetAsync(s->d_works, 0, 16 * sizeof(unsigned int), s->st));
@@ -1405,10 +1415,27 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   return DSM_OK;
 }
 
+int dsm::state_lost(dsm_sim* s) {
+  return fail(s, DSM_ERR_CUDA, "the chains of this ensemble were lost in an earlier launch: set them anew");
+}
+
+extern "C" int dsm_set_wait_polls(dsm_sim* s, uint32_t polls) {
+  if (!s || !s->ready || s->pending) return DSM_ERR_INVALID;
+  s->wait_polls = polls > 0 ? polls : kWaitPolls;
+  ++s->sched_version;  // (captured series hold the limit)
+  return DSM_OK;
+}
+
 // Status word of a launch: bit 0 aborted through the run flag, bit 1 a wait
-// between the warps of a block ran out
+// between the warps of a block ran out.  The chains that were resident then did
+// not come back: their vectors in HBM are not in strand order and belong to a
+// later time than the rest of their state, so the handle is of no use until its
+// chains are set anew.
 static int launch_status(dsm_sim* s, int status) {
-  if (status & 2) return fail(s, DSM_ERR_CUDA, "step kernel: a wait between warps ran out");
+  if (status & 2) {
+    s->lost = true;
+    return fail(s, DSM_ERR_CUDA, "step kernel: a wait between warps ran out; the chains of this ensemble are lost");
+  }
   return (status & 1) ? DSM_ABORTED : DSM_OK;
 }
 
@@ -1423,6 +1450,8 @@ static int series_collect(dsm_sim* s, dsm_stress_plus* out, uint64_t* events) {
   CK(cudaGetLastError());
   const int n = s->ser_n;
   const double* h_out = ser_out_h(s);
+  const int rc = launch_status(s, s->hw->status);
+  if (s->lost) return rc;
   const unsigned long long ev = s->hw->cnt[0];
   if (events) *events = ev;
   s->events_total += ev;
@@ -1433,7 +1462,7 @@ static int series_collect(dsm_sim* s, dsm_stress_plus* out, uint64_t* events) {
     for (int q = 0; q < 9; ++q) s->hw->red[q] = h_out[9 * (n - 1) + q];
     if (out) for (int w = 0; w < n; ++w) stress_out(h_out + 9 * w, &out[w]);
   }
-  return launch_status(s, s->hw->status);
+  return rc;
 }
 
 // wait for the pending work of s, forwarding the caller's abort flag
@@ -1458,6 +1487,7 @@ extern "C" int dsm_advance_series(dsm_sim* s, double dt, int32_t n, const volati
                                   dsm_stress_plus* out, uint64_t* events) {
   const dsm::NvtxRange nvtx_range("dsm_advance_series");
   if (!s || !s->ready || n < 1 || !(dt > 0.0) || s->pending) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   *s->h_abort = (abort_flag && *abort_flag) ? 1 : 0;
   const std::vector<double> e = series_ends(s, dt, n);
   int rc = series_start(s, e.data(), n);
@@ -1471,6 +1501,7 @@ extern "C" int dsm_advance_series(dsm_sim* s, double dt, int32_t n, const volati
 extern "C" int dsm_advance_start(dsm_sim* s, double t_end, int64_t step_limit) {
   const dsm::NvtxRange nvtx_range("dsm_advance_start");
   if (!s || !s->ready || s->pending) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   if (!(t_end >= 0.0) || t_end * TICKS >= 9.0e18) return fail(s, DSM_ERR_INVALID, "t_end out of range");
   *s->h_abort = 0;
   int rc = sim_launch_window(s, t_end, step_limit);
@@ -1482,6 +1513,7 @@ extern "C" int dsm_advance_start(dsm_sim* s, double t_end, int64_t step_limit) {
 extern "C" int dsm_series_start(dsm_sim* s, const double* t_ends, int32_t n) {
   const dsm::NvtxRange nvtx_range("dsm_series_start");
   if (!s || !s->ready || !t_ends || n < 1 || s->pending) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   *s->h_abort = 0;
   const int rc = series_start(s, t_ends, n);
   if (rc == DSM_OK) s->pending = 2;
@@ -1554,13 +1586,14 @@ static int enqueue_readback(dsm_sim* s) {
 static int window_collect(dsm_sim* s, uint64_t* events) {
   CK(cudaGetLastError());
   const unsigned long long* cnt = s->hw->cnt;
-  const int status = s->hw->status;
+  const int rc = launch_status(s, s->hw->status);
+  if (s->lost) return rc;
   if (events) *events = cnt[0];
   s->events_total += cnt[0];
   s->t_done = std::max(s->t_done, s->t_window);
   s->last_events = cnt[0];
   CK(cudaEventElapsedTime(&s->last_kernel_ms, s->ev0, s->ev1));
-  return launch_status(s, status);
+  return rc;
 }
 
 int dsm::sim_finish_window(dsm_sim* s, uint64_t* events) {
@@ -1574,6 +1607,7 @@ extern "C" int dsm_advance(dsm_sim* s, double t_end, int64_t step_limit, const v
                            uint64_t* events) {
   const dsm::NvtxRange nvtx_range("dsm_advance");
   if (!s || !s->ready) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   if (!(t_end >= 0.0) || t_end * TICKS >= 9.0e18) return fail(s, DSM_ERR_INVALID, "t_end out of range");
   *s->h_abort = (abort_flag && *abort_flag) ? 1 : 0;
   if (s->pending) return fail(s, DSM_ERR_INVALID, "an asynchronous advance is pending (dsm_poll it first)");
@@ -1588,6 +1622,7 @@ extern "C" int dsm_advance(dsm_sim* s, double t_end, int64_t step_limit, const v
 
 extern "C" int dsm_stress(dsm_sim* s, dsm_stress_plus* out, int32_t* count) {
   if (!s || !s->ready || !out) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   if (!s->flow) {
     // equilibrium ensembles keep no per-chain stress: evaluate it from the
     // current state, with the sums and the reduction of a flow window end
@@ -1611,6 +1646,7 @@ extern "C" int dsm_stress(dsm_sim* s, dsm_stress_plus* out, int32_t* count) {
 extern "C" int dsm_gt_raw(dsm_sim* s, double* gsum, int64_t* count) {
   const dsm::NvtxRange nvtx_range("dsm_gt_raw");
   if (!s || !s->ready) return DSM_ERR_INVALID;
+  if (s->lost) return state_lost(s);
   if (!s->corr) return fail(s, DSM_ERR_INVALID, "no correlator in this simulation (eq_type != 1 or flow)");
   const size_t m = (size_t)s->levels * s->cp;
   CK(launch_gt_reduce_dev(s->d_ens, s->levels, s->cp, s->d_gsum, s->d_gcnt, s->st));
@@ -1717,6 +1753,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   if (!s || !s->ready) return DSM_ERR_INVALID;
   for (int i = 0; i < n; ++i) {
     if (!sims[i] || !sims[i]->ready) return DSM_ERR_INVALID;
+    if (sims[i]->lost) return state_lost(s);
     if (sims[i]->pending) return fail(s, DSM_ERR_INVALID, "an ensemble of the batch has asynchronous work pending");
     if (sims[i]->P.device != s->P.device) return fail(s, DSM_ERR_INVALID, "batch spans devices");
     if (!(t_end[i] >= 0.0) || t_end[i] * TICKS >= 9.0e18) return fail(s, DSM_ERR_INVALID, "t_end out of range");
@@ -1773,7 +1810,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   std::vector<cudaStream_t> used;
   cudaEvent_t ready = nullptr;
   std::vector<cudaEvent_t> joins;
-  std::vector<std::pair<int, int*>> words;  // first ensemble of a group, its launch's status word
+  std::vector<int*> words;  // status word of each group's launch
   const bool fan = groups.size() > 1;
   auto enqueue = [&]() -> int {
     if (fan) {
@@ -1856,12 +1893,13 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
         lst.defer = dDef;
         lst.n_defer = dW + 2;
       }
+      lst.polls = sims[g.idx[0]]->wait_polls;
       if (fan) {
         CK(cudaEventRecord(ready, s->st));
         CK(cudaStreamWaitEvent(gs, ready, 0));
       }
       used.push_back(gs);
-      words.push_back({g.idx[0], (int*)(dW + 1)});
+      words.push_back((int*)(dW + 1));
       CK(launch_step(dE, k, dP, pre[k], dW, g.flow, g.corr, run, nullptr, (int*)(dW + 1), grid, gs, lst));
       if (overflow) {
         StepList ol;
@@ -1885,8 +1923,8 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
       }
       CK(cudaMemcpyAsync(q->hw->cnt, q->d_counters, sizeof(q->hw->cnt), cudaMemcpyDeviceToHost, s->st));
     }
-    for (const auto& w : words)
-      CK(cudaMemcpyAsync(&sims[w.first]->hw->status, w.second, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    for (size_t g = 0; g < groups.size(); ++g)
+      CK(cudaMemcpyAsync(&sims[groups[g].idx[0]]->hw->status, words[g], sizeof(int), cudaMemcpyDeviceToHost, s->st));
     return DSM_OK;
   };
   const int rc = enqueue();
@@ -1902,14 +1940,18 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   if (sync_err != cudaSuccess)
     return fail(s, DSM_ERR_CUDA, std::string("dsm_advance_batch: ") + cudaGetErrorString(sync_err));
   CK(cudaGetLastError());
-  for (const auto& w : words)
-    if (const int st = launch_status(s, sims[w.first]->hw->status)) return st;
+  int status = DSM_OK;
+  for (const auto& g : groups)
+    for (const int i : g.idx)
+      if (const int st = launch_status(sims[i], sims[g.idx[0]]->hw->status)) status = st;
   for (int i = 0; i < n; ++i) {
+    if (sims[i]->lost) continue;
     const unsigned long long* cnt = sims[i]->hw->cnt;
     if (events) events[i] = cnt[0];
     sims[i]->events_total += cnt[0];
     sims[i]->last_events = cnt[0];
     sims[i]->t_done = std::max(sims[i]->t_done, sims[i]->t_window);
   }
-  return DSM_OK;
+  if (status != DSM_OK && !s->lost) fail(s, status, "a wait between warps ran out; an ensemble of the batch is lost");
+  return status;
 }

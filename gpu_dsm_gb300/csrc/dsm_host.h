@@ -147,6 +147,8 @@ struct dsm_sim {
   // time slices of a launch (EnsDev::subs): the most that pay for this plan, and
   // their per-chain words
   int sub_max = 1;
+  unsigned wait_polls = dsm::kWaitPolls;  // StepList::polls
+  bool lost = false;  // a launch gave up with chains resident: refuse what reads them until they are set anew
   dsm::Slice* d_slice = nullptr;
   cudaStream_t side = nullptr, side2 = nullptr, side3 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
@@ -172,6 +174,8 @@ int plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float margi
 // carved form of a class plan (dsm_set_class_form) in blocks of block_smem
 // bytes; leaves the plan as it is if a class's slot does not fit the block
 int plan_carve(dsm_sim* s, const SizeClass& big, const SizeClass& mid, const SizeClass& small, size_t block_smem);
+// the error of a call that needs the chains of a lost ensemble
+int state_lost(dsm_sim* s);
 int sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit);
 int sim_finish_window(dsm_sim* s, uint64_t* events);
 }  // namespace dsm

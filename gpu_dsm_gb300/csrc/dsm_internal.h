@@ -104,7 +104,9 @@ struct EnsDev {
   float2* corr_comp;
   float* corr_buf;                 // [chain][kCorrBuf][3] samples of the running launch not yet correlated
   float* out_stress;               // [chain][8] stress at the end of the launch (flow)
-  unsigned long long* counters;    // [0] events this launch, [1] chains done
+  // [0] events this launch, [1] chains done, [2] chains deferred, [3] lockstep
+  // launches (of the first ensemble): times a chain's event counter passed 4096 more
+  unsigned long long* counters;
   // flow output series inside one launch (n_win > 0): window w ends at
   // win[w] ticks with event cap win[win_stride + w]; a chain records its stress
   // at each window end in win_stress[w][chain][8] and keeps running; its next
@@ -116,6 +118,7 @@ struct EnsDev {
 
 constexpr int kCorrBuf = 64;  // samples of a chain that the lockstep kernel correlates at a time
 constexpr int kCarveMax = 4;  // size classes of one carved launch
+constexpr unsigned kWaitPolls = 1u << 28;  // StepList::polls: half a minute or so
 
 struct LaunchCfg {
   int warps_per_block;
@@ -161,6 +164,9 @@ struct StepList {
   int carve_first[kCarveMax] = {};
   int carve_count[kCarveMax] = {};
   unsigned int* carve_work = nullptr;
+  // polls of a wait between the warps of a block after which it gives up if the
+  // launch made no progress meanwhile (lockstep kernel; status bit 1)
+  unsigned int polls = kWaitPolls;
 };
 
 // kernels (dsm_kernels.cu)

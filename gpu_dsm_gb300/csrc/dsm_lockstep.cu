@@ -66,9 +66,10 @@ struct LCorr : Corr0 {
   long long nbuf;  // samples in the chain's buffer
 };
 
-// Request and completion bits of a block's slots, and the number of requests served
+// Request and completion bits of a block's slots; per warp, what lock_moved saw last
 struct Ctl {
-  unsigned req, done, dead, served;
+  unsigned req, done, dead, pad_;
+  unsigned seen[4];
 };
 
 // Shared-memory slot of one chain.  The strand vectors Q stay in HBM (L2), in
@@ -83,7 +84,7 @@ struct LSlot {
 };
 
 constexpr size_t kLockHead = (sizeof(Hdr) + sizeof(LCorr) + 15) / 16 * 16;  // C is read 16 bytes at a time
-static_assert(sizeof(Hdr) % 16 == 0 && sizeof(Ctl) == 16, "slot alignment");
+static_assert(sizeof(Hdr) % 16 == 0 && sizeof(Ctl) == 32, "slot alignment");
 
 __host__ __device__ inline size_t lock_bytes(int slot_cap, int subs, int sb) {
   size_t b = ((size_t)slot_cap + 1) * 16 + kLockHead;
@@ -616,6 +617,13 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
   return code;
 }
 
+// Every 4096 events of a chain: a sign that the launch moves (lock_moved), and
+// whether it is to be aborted
+__device__ __noinline__ bool lock_look(const EnsDev* ens, const volatile int* abort_flag) {
+  if ((threadIdx.x & 31) == 0) atomicAdd(&ens[0].counters[3], 1ull);
+  return abort_flag != nullptr && wshfl(*abort_flag, 0) != 0;
+}
+
 // Everything a chain needs before its next slide, by one service warp: the
 // requested event, due samples, the way back to HBM and the next chain, rate
 // passes, the prefix of the pair totals.  False: the slot's next chain is not back
@@ -644,7 +652,7 @@ __device__ __forceinline__ bool lock_serve(const EnsDev* __restrict__ ens, int n
     hash = (hash ^ (uint64_t)code) * 0x100000001B3ull;
     ++step;
   }
-  if (live && abort_flag != nullptr && (step & 4095) == 0) aborted = wshfl(*abort_flag, 0) != 0;
+  if (live && (step & 4095) == 0) aborted = lock_look(ens, abort_flag);
 #pragma unroll 1
   for (;;) {
     if (live) {
@@ -893,7 +901,19 @@ __global__ void __launch_bounds__(128) k_slice_flush(const EnsDev* __restrict__ 
   if (lane == 0) lock_corr_store(E, c, *k0);
 }
 
-constexpr unsigned kSpinLimit = 1u << 28;  // polls of a wait before it gives up (status bit 1)
+// Whether the launch has moved since the warp last asked: a chain taken from the
+// work list or 4096 more events of one.  A wait that has polled StepList::polls
+// times goes on if so (a chain's earlier time slice may run for minutes in another
+// block), else gives up (status bit 1).
+__device__ __noinline__ bool lock_moved(const EnsDev* ens, const unsigned int* work, unsigned* seen) {
+  int moved = 0;
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned n = *(const volatile unsigned int*)work + (unsigned)*(const volatile unsigned long long*)&ens[0].counters[3];
+    moved = n != *seen;
+    *seen = n;
+  }
+  return wshfl(moved, 0) != 0;
+}
 
 template <int CK, int G, int SB, int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens, int n_ens,
@@ -920,7 +940,8 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
         s.h->pend = 0;
       }
     }
-    if (threadIdx.x == 0) { ctl->req = all; ctl->done = 0u; ctl->dead = 0u; ctl->served = 0u; }
+    if (threadIdx.x == 0) { ctl->req = all; ctl->done = 0u; ctl->dead = 0u; }
+    if (threadIdx.x < 4) ctl->seen[threadIdx.x] = 0u;
   }
   __syncthreads();
 
@@ -928,7 +949,7 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     // ------------------------------------------------ service warp
     const long long n_items = lst.dyn_total != nullptr ? (long long)*lst.dyn_total : total;
     const int subs = lst.dyn_total != nullptr ? 1 : ens[0].subs;  // time slices
-    unsigned idle = 0, seen = 0, waits = 0, turn = ~0u;
+    unsigned idle = 0, turn = ~0u;  // polls since this warp last served a request
     for (;;) {
       int b = -1;
       if (lane == 0) {
@@ -946,39 +967,32 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
       }
       b = wshfl(b, 0);
       if (b == -3) return;
-      if (b < 0) {
-        if (++idle > kSpinLimit) {
-          // no request came: give up unless the block's other warps served some
-          const unsigned n = wshfl(*(volatile unsigned*)&ctl->served, 0);
-          if (n == seen) {
-            if (lane == 0) atomicOr(status, 2);
-            return;
-          }
-          seen = n;
-          idle = 0;
-        }
-        if (b == -1) __nanosleep(100);
-        continue;
-      }
-      idle = 0;
-      // what the slide lanes wrote before the request, seen by lane 0, now by all
-      __threadfence_block();
-      __syncwarp();
-      const LSlot sl = lock_slot(slots + (size_t)b * sbytes, slot_cap, SB);
-      const bool done = lock_serve<CK, SUBS, SB>(ens, n_ens, prefix, n_items, subs, work, slot_cap, sl, 1u << b, ctl,
-                                                 abort_flag, status, lst);
-      __syncwarp();
-      if (lane == 0) {
-        if (done) atomicAdd(&ctl->served, 1u);
+      if (b >= 0) {
+        // what the slide lanes wrote before the request, seen by lane 0, now by all
         __threadfence_block();
-        atomicOr(done ? &ctl->done : &ctl->req, 1u << b);
+        __syncwarp();
+        const LSlot sl = lock_slot(slots + (size_t)b * sbytes, slot_cap, SB);
+        const bool done = lock_serve<CK, SUBS, SB>(ens, n_ens, prefix, n_items, subs, work, slot_cap, sl, 1u << b, ctl,
+                                                   abort_flag, status, lst);
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence_block();
+          atomicOr(done ? &ctl->done : &ctl->req, 1u << b);
+        }
+        if (done) {
+          idle = 0;
+          continue;
+        }
       }
-      waits = done ? 0u : waits + 1u;
-      if (waits > kSpinLimit) {
-        if (lane == 0) atomicOr(status, 2);
-        return;
+      if (++idle > lst.polls) {
+        if (!lock_moved(ens, work, &ctl->seen[warp])) {
+          if (lane == 0) atomicOr(status, 2);
+          return;
+        }
+        idle = 0;
       }
-      if (!done) __nanosleep(1000);
+      if (b == -1) __nanosleep(100);
+      else if (b >= 0) __nanosleep(1000);
     }
   }
 
@@ -1042,9 +1056,12 @@ __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens,
     }
     if (!__any_sync(FULL_MASK, run)) {
       if (__all_sync(FULL_MASK, dead)) return;
-      if (++idle > kSpinLimit) {
-        if (lane == 0) atomicOr(status, 2);
-        return;
+      if (++idle > lst.polls) {
+        if (!lock_moved(ens, work, &ctl->seen[warp])) {
+          if (lane == 0) atomicOr(status, 2);
+          return;
+        }
+        idle = 0;
       }
       __nanosleep(20);
       continue;

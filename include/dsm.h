@@ -248,6 +248,13 @@ int dsm_get_class_form(const dsm_sim* sim, int32_t* form);
  * reference (fixed launch shapes). */
 int dsm_autotune(dsm_sim* sim, double window, int32_t* best, float* best_ms);
 
+/* Polls, without progress anywhere in the launch, after which a wait between the
+ * warps of a lockstep launch gives up (0: the default, 2^28 polls, half a minute or so).  The advance
+ * then returns DSM_ERR_CUDA and the clock stays where it was; the chains are
+ * lost, and calls that need them return DSM_ERR_CUDA until they are set anew
+ * (dsm_set_chains, dsm_init_equilibrium, dsm_load_file, dsm_checkpoint_load). */
+int dsm_set_wait_polls(dsm_sim* sim, uint32_t polls);
+
 /* Counters of the last window: kMC events, chains that completed the window
  * in their first slot, chains moved to a larger slot on the way. */
 int dsm_window_stats(const dsm_sim* sim, uint64_t* events, uint64_t* chains_done, uint64_t* deferred);
