@@ -144,6 +144,8 @@ def load_library() -> C.CDLL:
     lib.dsm_get_schedule.restype = C.c_int
     lib.dsm_set_wait_polls.argtypes = [vp, C.c_uint32]
     lib.dsm_set_wait_polls.restype = C.c_int
+    lib.dsm_get_step_kernel.argtypes = [vp, vp]
+    lib.dsm_get_step_kernel.restype = C.c_int
     lib.dsm_set_class_form.argtypes = [vp, i32]
     lib.dsm_set_class_form.restype = C.c_int
     lib.dsm_get_class_form.argtypes = [vp, C.POINTER(i32)]
@@ -478,6 +480,13 @@ class Ensemble:
         keys = ("slot", "warps_per_block", "lanes", "grid", "chains")
         m = n.value + 1 if n.value else 0
         return [dict(zip(keys, info[5 * i:5 * i + 5].tolist())) for i in range(m)]
+
+    def step_kernel(self) -> dict:
+        """Step kernel of the last (or only) class: lockstep or tiles, lanes per chain,
+        strands of a slot, time slices of the last launch (dsm_get_step_kernel)."""
+        info = np.zeros(4, np.int32)
+        self._check(self._lib.dsm_get_step_kernel(self._h, _ptr(info)))
+        return {"lockstep": bool(info[0]), "lanes": int(info[1]), "slot": int(info[2]), "slices": int(info[3])}
 
     def save(self, path: str) -> None:
         self._check(self._lib.dsm_save_file(self._h, os.fsencode(path)))

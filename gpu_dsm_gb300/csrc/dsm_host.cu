@@ -1011,6 +1011,18 @@ extern "C" int dsm_get_schedule(const dsm_sim* s, int32_t* n_classes, int32_t* i
   return DSM_OK;
 }
 
+extern "C" int dsm_get_step_kernel(const dsm_sim* s, int32_t* info) {
+  if (!s || !s->ready || !info) return DSM_ERR_INVALID;
+  LaunchCfg c = s->classes.empty() ? s->cfg : s->classes.back().cfg;
+  if (s->carved) c.lock = false;
+  const bool lock = c.lock && !s->flow && lock_lanes(c.slot_cap) != 0;
+  info[0] = lock ? 1 : 0;
+  info[1] = lock ? lock_lanes(c.slot_cap) : c.lanes;
+  info[2] = c.slot_cap;
+  info[3] = s->h.subs;
+  return DSM_OK;
+}
+
 extern "C" int dsm_corr_shape(const dsm_sim* s, int32_t* levels, int32_t* p, int32_t* m) {
   if (!s) return DSM_ERR_INVALID;
   if (levels) *levels = s->corr ? s->levels : 0;

@@ -220,6 +220,10 @@ int dsm_set_schedule(dsm_sim* sim, int32_t small_slot, int32_t large_grid, int32
 #define DSM_SCHEDULE_INFO 25
 int dsm_get_schedule(const dsm_sim* sim, int32_t* n_classes, int32_t* info);
 
+/* Step kernel of the plan's last (or only) class: info = {1 lockstep or 0 tiles,
+ * lanes per chain, slot strands, time slices of the last launch}. */
+int dsm_get_step_kernel(const dsm_sim* sim, int32_t info[4]);
+
 /* How size classes launch (equilibrium ensembles whose small class runs 16
  * lanes per chain).  form 0 (default): each class its own persistent launch,
  * the four launched concurrently on four streams.  form 1: the large, middle

@@ -1,0 +1,135 @@
+"""Which ensembles the lockstep kernel runs, with how many lanes and time slices (the
+bit-for-bit tests of that kernel hold only where it is the one that runs), and its
+plans in the other ways to advance: batches, captured series, saved states, an
+abort between two slices."""
+import threading
+
+import numpy as np
+import pytest
+
+from helpers import assert_bitexact, gpu_state
+
+pytestmark = pytest.mark.gpu
+N = 7400
+TICKS = 2.0**32
+SLICED = dict(nk=300, beta=0.5, n_chains=6000)
+
+
+def gt(p, m, **kw):
+    return dict(eq_type=1, corr_p=p, corr_m=m, sync_dt=0.25, t_end=4000.0, **kw)
+
+
+def same_run(a, b, times, what):
+    for t in times:
+        assert a.advance(t) == b.advance(t)
+    assert_bitexact(gpu_state(a), gpu_state(b), what=what)
+
+
+@pytest.mark.parametrize("kw,lanes", [
+    (dict(nk=100, beta=10.0), 4), (dict(nk=90, beta=3.0), 4), (dict(nk=100), 4), (dict(nk=131), 4),
+    (dict(nk=170, beta=0.5), 8), (dict(nk=463, beta=0.5), 8), (dict(nk=100, cd_flag=0), 4), (dict(nk=100, z_max=52), 4),
+    (dict(nk=100, gex=(1.0, 1.0, 1000.0, 100.0)), 4), (gt(16, 2, nk=151), 4), (gt(64, 8, nk=200), 4),
+    (gt(96, 4, nk=204, beta=0.5), 8), (dict(gt(8, 2, nk=151), eq_type=2), 4), (dict(nk=100, beta=100.0), 4)], ids=str)
+def test_kernel_of_the_plan(dsm_mod, kw, lanes):
+    k = dsm_mod.Ensemble(n_chains=N, seed=71, **kw).step_kernel()
+    assert k["lockstep"] and k["lanes"] == lanes
+
+
+@pytest.mark.parametrize("kw", [dict(nk=20), dict(nk=200, lanes_per_chain=16), dict(nk=200, lanes_per_chain=32),
+                                dict(nk=200, kappa=(0.0, 2.0e-3) + (0.0,) * 7)], ids=str)
+def test_tiles_otherwise(dsm_mod, kw):
+    assert not dsm_mod.Ensemble(n_chains=N, seed=71, **kw).step_kernel()["lockstep"]
+    assert not dsm_mod.Ensemble(n_chains=900, nk=200, seed=71).step_kernel()["lockstep"]
+
+
+def test_slices_of_a_launch(dsm_mod):
+    e = dsm_mod.Ensemble(seed=74, **SLICED)
+    e.init_equilibrium()
+    e.advance(55.0)
+    assert e.step_kernel() == {"lockstep": True, "lanes": 8, "slot": e.step_kernel()["slot"], "slices": 4}
+    e.advance(55.5)  # a few dozen events per chain
+    assert e.step_kernel()["slices"] == 1
+
+
+def test_batch_of_lockstep_ensembles(dsm_mod):
+    """Two lockstep ensembles in one launch, beside groups of other kernels."""
+    kws = [dict(gt(64, 8, nk=200), n_chains=N), dict(gt(64, 8, nk=160), n_chains=8000), dict(nk=170, n_chains=N),
+           dict(gt(64, 8, nk=200), n_chains=900), dict(nk=30, n_chains=500)]
+    a = [dsm_mod.Ensemble(seed=76, stream=i, **k) for i, k in enumerate(kws)]
+    b = [dsm_mod.Ensemble(seed=76, stream=i, lanes_per_chain=16, **k) for i, k in enumerate(kws)]
+    assert [x.step_kernel()["lockstep"] for x in a] == [True, True, True, False, False]
+    for x in a + b:
+        x.init_equilibrium()
+    for t in (1.5, 4.0):
+        ev = dsm_mod.advance_batch(a, t)
+        assert list(ev) == [x.advance(t) for x in b]
+    for x, y in zip(a, b):
+        assert_bitexact(gpu_state(x), gpu_state(y), what="batch")
+    # (chains of the first outgrow the group's slot, which is the second's: their
+    # level-0 sums are cut in two FP32 pieces there, in tiles as here)
+    assert a[0].window_stats()["deferred"] > 0 == a[1].window_stats()["deferred"]
+    assert np.array_equal(a[0].gt_raw()[1], b[0].gt_raw()[1])
+    assert np.array_equal(a[1].gt_raw()[0], b[1].gt_raw()[0])
+
+
+@pytest.mark.parametrize("z_max", [0, 52], ids=["classes", "captured"])
+def test_series(dsm_mod, z_max):
+    """An equilibrium series: size classes issue its windows, a plan of one launch
+    replays them from a captured graph."""
+    kw = dict(nk=100, z_max=z_max, n_chains=N, seed=77)
+    a, b = dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(lanes_per_chain=16, **kw)
+    assert a.step_kernel()["lockstep"] and (a.schedule() == []) == (z_max > 0)
+    for x in (a, b):
+        x.init_equilibrium()
+    for _ in range(2):
+        assert a.advance_series(0.5, 3)[0] == b.advance_series(0.5, 3)[0]
+    assert_bitexact(gpu_state(a), gpu_state(b), what="series")
+
+
+def test_saved_and_reloaded(dsm_mod, tmp_path):
+    kw = dict(gt(64, 8, nk=200), n_chains=N, seed=78)
+    a, b, c = dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(lanes_per_chain=16, **kw)
+    a.init_equilibrium()
+    a.advance(3.0)
+    a.checkpoint(str(tmp_path / "k"))
+    for x in (b, c):
+        x.restore(str(tmp_path / "k"))
+    assert b.step_kernel()["lockstep"]
+    a.advance(8.0)
+    same_run(b, c, [8.0], "restored")
+    assert_bitexact(gpu_state(a), gpu_state(b), what="continued")
+    assert np.array_equal(a.gt_raw()[0], b.gt_raw()[0]) and np.array_equal(b.gt_raw()[0], c.gt_raw()[0])
+    a.save(str(tmp_path / "c"))
+    for x in (b, c):
+        x.load(str(tmp_path / "c"))
+    same_run(b, c, [10.0], "loaded")
+
+
+def test_abort_between_two_slices(dsm_mod):
+    """Told to abort while some chains wait between two slices: they stopped at the end
+    of one, and no sample is lost."""
+    kw = dict(gt(64, 8, **SLICED), seed=75)
+    a, b = dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    flag = np.zeros(1, np.int32)
+    timer = threading.Timer(0.25, lambda: flag.__setitem__(0, 1))
+    timer.start()
+    end = 3000.0
+    assert a.advance(end, abort=flag) == -1
+    timer.join()
+    k = a.step_kernel()["slices"]
+    assert k > 1
+    T = a.get_ext()["T"] / TICKS
+    done = np.floor(T / (end / k) + 1e-9).astype(int)  # slices each chain has finished
+    assert done.max() >= 1 and T.min() < end
+    stopped = (done >= 1) & (done < k) & (T - done * (end / k) < 1.0)  # just past a slice's end
+    assert stopped.sum() > 50
+    assert a.advance(end) != -1
+    b.advance(end)
+    ga, ca = a.gt_raw()
+    gb, cb = b.gt_raw()
+    assert np.array_equal(ca, cb)
+    # a sum cut in two FP32 compensated pieces where the abort fell
+    assert np.abs(ga - gb).max() <= 2.0**-22 * np.abs(gb).max()
+    assert_bitexact(gpu_state(a), gpu_state(b), what="abort between slices")
