@@ -1408,6 +1408,7 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   for (int w = 0; w < n; ++w) {
     h_win[w] = (long long)std::llrint(ends[w] * TICKS);  // as dsm_advance(ends[w])
     h_win[s->ser_cap + w] = (long long)window_watchdog(s, ends[w] - t_prev);
+    shortest = std::min(shortest, ends[w] - t_prev);
     t_prev = ends[w];
   }
   s->t_window = t_prev;

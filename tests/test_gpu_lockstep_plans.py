@@ -51,6 +51,22 @@ def test_slices_of_a_launch(dsm_mod):
     assert e.step_kernel()["slices"] == 1
 
 
+@pytest.mark.parametrize("ends,slices", [((80.0, 81.0, 161.0), 1), ((80.0, 160.0, 240.0), 4)], ids=str)
+def test_slices_of_a_series(dsm_mod, ends, slices):
+    """The shortest window of a series decides: slices of a window of a few dozen events
+    would load and store every chain for a handful of them."""
+    a, b = (dsm_mod.Ensemble(seed=79, lanes_per_chain=k, **SLICED) for k in (0, 16))
+    for x in (a, b):
+        x.init_equilibrium()
+    a.series_start(ends)
+    while a.poll() is None:
+        pass
+    assert a.step_kernel()["lockstep"] and a.step_kernel()["slices"] == slices
+    for t in ends:
+        b.advance(t)
+    assert_bitexact(gpu_state(a), gpu_state(b), what="series")
+
+
 def test_batch_of_lockstep_ensembles(dsm_mod):
     """Two lockstep ensembles in one launch, beside groups of other kernels."""
     kws = [dict(gt(64, 8, nk=200), n_chains=N), dict(gt(64, 8, nk=160), n_chains=8000), dict(nk=170, n_chains=N),
