@@ -536,6 +536,11 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
   LaunchCfg sc = s->cfg;
   if (lanes == 16 || lanes == 32) sc.lanes = lanes;
   sc.warps_per_block = 4;
+  // (slots are sized by the tiles, whose kernel the carved form runs; a lockstep
+  // plan comes with its slot)
+  const bool lock = s->cfg.lock;
+  sc.lock = false;
+  sc.tiles = 0;
   // full occupancy of the step kernel is 4 blocks x 4 warps per SM (register bound)
   const int full_cap = largest_slot(s->flow, s->ck, sc, 4, s->cap);
   if (small_cap <= 0) small_cap = full_cap;
@@ -624,7 +629,7 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
     // with the small one for block slots, and a work-share grid left it
     // finishing alone at the end of every window (measured 9.6e8 vs 1.2e9
     // events/s on the 262144-chain log-normal melt)
-    M.cfg = LaunchCfg{4, mid_cap, s->cfg.pmax, 32, s->cfg.lock};
+    M.cfg = LaunchCfg{4, mid_cap, s->cfg.pmax, 32, lock};
     const int lb = plan_lock(s, M.cfg, (long long)mid.size());
     M.bps = step_max_blocks_per_sm(s->flow, s->ck, M.cfg);
     if (lb > 0) M.bps = std::min(M.bps, lb);
@@ -634,7 +639,7 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
     M.count = (long long)mid.size();
     M.grid = (int)std::max<long long>(1, std::min<long long>((M.count + mt - 1) / mt, (long long)M.bps * s->sm_count));
   }
-  Sm.cfg = LaunchCfg{4, small_cap, s->cfg.pmax, sc.lanes, s->cfg.lock};
+  Sm.cfg = LaunchCfg{4, small_cap, s->cfg.pmax, sc.lanes, lock};
   const int small_lb = plan_lock(s, Sm.cfg, (long long)small.size());
   Sm.bps = step_max_blocks_per_sm(s->flow, s->ck, Sm.cfg);
   if (small_lb > 0) Sm.bps = std::min(Sm.bps, small_lb);
@@ -660,7 +665,6 @@ int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float 
   if (s->carve && !s->flow && sc.lanes == 16) {
     LaunchCfg full = sc;
     full.slot_cap = full_cap;
-    full.lock = false;
     plan_carve(s, B, M, Sm, step_block_smem(false, full));
   }
   return plan_buffers(s);
@@ -785,9 +789,13 @@ static int tile_schedule(dsm_sim* s) {
 // Its slot is the smallest that holds the chains' bound, so that as many chains as
 // possible are resident.
 static int default_schedule(dsm_sim* s) {
+  s->by_default = true;
+  s->cfg.lock = false;
+  s->cfg.lanes = s->P.lanes_per_chain > 0 ? s->P.lanes_per_chain : 32;
+  s->cfg.warps_per_block = std::min(4, s->P.warps_per_block > 0 ? s->P.warps_per_block : 4);
   if (s->P.lanes_per_chain != 0) return plan_single(s);
   const int rc = tile_schedule(s);
-  if (rc != DSM_OK || !prefer_lock(s)) return rc;
+  if (rc != DSM_OK || s->carve || !prefer_lock(s)) return rc;
   const LaunchCfg& t = s->classes.empty() ? s->cfg : s->classes.back().cfg;
   if ((long long)s->P.n_chains <= (long long)s->blocks_per_sm * s->sm_count * step_tiles(s->flow, t)) return rc;
   const double pe = 1.0 / (1.0 + (double)s->P.beta), nk = (double)s->P.nk;
@@ -795,7 +803,7 @@ static int default_schedule(dsm_sim* s) {
   const int slot = std::max(8, (int)std::ceil(zb));
   if (lock_lanes(std::min(slot, s->cap)) == 0) return rc;
   s->cfg.lanes = 16;
-  s->cfg.lock = true;
+  s->cfg.lock = s->lock_default = true;
   return slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
 }
 
@@ -871,7 +879,14 @@ extern "C" int dsm_set_schedule(dsm_sim* s, int32_t small_slot, int32_t large_gr
   if (lanes != 0 && lanes != 16 && lanes != 32) return fail(s, DSM_ERR_INVALID, "lanes must be 16 or 32");
   CK(cudaStreamSynchronize(s->st));
   small_schedule_end(s);
-  if (lanes) { s->cfg.lanes = lanes; s->cfg.lock = false; }
+  // the handle's own kernel again (also after tiles were chosen)
+  if (lanes == 0 && s->lock_default) {
+    if (small_slot <= 0) return default_schedule(s);
+    s->cfg.lanes = 16;
+  }
+  s->cfg.lock = lanes == 0 && s->lock_default && !s->carve;
+  s->by_default = false;
+  if (lanes) s->cfg.lanes = lanes;
   // monodisperse ensembles keep one launch with full-capacity slots unless a
   // smaller slot is asked for (chains that outgrow it finish in the overflow launch)
   if (!s->poly && small_slot <= 0) return plan_single(s);
@@ -882,6 +897,13 @@ extern "C" int dsm_set_class_form(dsm_sim* s, int32_t form) {
   if (!s || !s->ready || (form != 0 && form != 1) || s->pending) return DSM_ERR_INVALID;
   CK(cudaStreamSynchronize(s->st));
   s->carve = form == 1;
+  // a default plan: the carved form runs the classes of 16-lane tiles, whatever the
+  // ensemble's number of chains makes of them otherwise
+  if (s->by_default && s->P.lanes_per_chain == 0) {
+    small_schedule_end(s);
+    const int rc = default_schedule(s);
+    return rc != DSM_OK || s->carve ? rc : small_schedule(s);
+  }
   if (s->classes.empty()) return DSM_OK;
   // the same classes again, in the form asked for
   int small = 0, grid = 0;
@@ -908,8 +930,11 @@ extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* bes
   if (!s || !s->ready || !(window > 0.0) || s->pending) return DSM_ERR_INVALID;
   if (s->lost) return state_lost(s);
   small_schedule_end(s);
+  // lanes 0: the plan that the ensemble starts with, where that is the lockstep kernel
   struct Cand { int small, grid, lanes, carve = 0; };
   std::vector<Cand> cands;
+  if (s->lock_default) cands.push_back({0, 0, 0});
+  s->cfg.lock = s->by_default = false;
   for (int lanes : {32, 16}) {
     if (!s->poly) cands.push_back({0, 0, lanes});  // one launch, full-capacity slots
     // small slot: the largest with 4, 3 or 2 blocks of 4 warps per SM
@@ -940,14 +965,19 @@ extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* bes
     }
   }
   const bool carve0 = s->carve;
+  auto plan_cand = [&](const Cand& c) {
+    s->carve = c.carve != 0;
+    if (c.lanes == 0) return default_schedule(s);
+    s->cfg.lanes = c.lanes;
+    s->cfg.lock = s->by_default = false;
+    return (s->poly || c.small > 0) ? plan_classes(s, c.small, c.grid, c.lanes, 0.f) : plan_single(s);
+  };
   int bi = -1;
   double brate = 0.0;
   float bms = 0.f;
   for (size_t i = 0; i < cands.size(); ++i) {
     const Cand& c = cands[i];
-    s->cfg.lanes = c.lanes;
-    s->carve = c.carve != 0;
-    int rc = (s->poly || c.small > 0) ? plan_classes(s, c.small, c.grid, c.lanes, 0.f) : plan_single(s);
+    int rc = plan_cand(c);
     if (rc != DSM_OK) return rc;
     rc = sim_launch_window(s, s->t_done + window, -1);
     if (rc == DSM_OK) rc = sim_finish_window(s, nullptr);
@@ -959,16 +989,17 @@ extern "C" int dsm_autotune(dsm_sim* s, double window, int32_t* best, float* bes
     // windows of a few tau_K came out within a few percent of each other.  So
     // a change of tile width must win its trial by kLaneMargin: 32 lanes must
     // be that much faster than the best 16-lane schedule, and 16 lanes may be
-    // that much slower than the best 32-lane one.
+    // that much slower than the best 32-lane one.  Against the lockstep default
+    // both must be that much faster.
     constexpr double kLaneMargin = 0.03;
     double need = brate;
-    if (bi >= 0 && c.lanes != cands[bi].lanes) need = brate * (c.lanes == 16 ? 1.0 - kLaneMargin : 1.0 + kLaneMargin);
+    if (bi >= 0 && c.lanes != cands[bi].lanes)
+      need = brate * (c.lanes == 16 && cands[bi].lanes != 0 ? 1.0 - kLaneMargin : 1.0 + kLaneMargin);
     if (bi < 0 || rate > need) { bi = (int)i; brate = rate; bms = s->last_kernel_ms; }
   }
-  const Cand& b = cands[bi];
-  s->cfg.lanes = b.lanes;
-  s->carve = b.carve != 0 || (carve0 && !s->poly);
-  const int rc = (s->poly || b.small > 0) ? plan_classes(s, b.small, b.grid, b.lanes, 0.f) : plan_single(s);
+  Cand b = cands[bi];
+  if (carve0 && !s->poly && b.lanes != 0) b.carve = 1;
+  const int rc = plan_cand(b);
   if (best) { best[0] = b.small; best[1] = b.grid; best[2] = b.lanes; best[3] = (int32_t)cands.size(); }
   if (best_ms) *best_ms = bms;
   return rc;

@@ -141,6 +141,8 @@ struct dsm_sim {
   size_t carve_smem = 0;
   bool shared = false;     // runs next to other ensembles on the device (dsm_server)
   bool lock_fits = false;  // device memory for the lockstep kernel's buffers
+  bool lock_default = false;  // the lockstep kernel is this ensemble's default (default_schedule)
+  bool by_default = false;    // monodisperse: the plan is the default one, not one that was asked for
   // one chain per warp because all chains are resident so (small_schedule): the
   // slot of the two-per-warp plan, which a batch of such ensembles may need; else 0
   int slot16 = 0;

@@ -209,8 +209,9 @@ int dsm_pcd(double beta, int32_t nk, double* out);
  * G(t) to the bit; the MSD centre-of-mass sums to rounding).  Arguments <= 0 choose
  * the defaults (largest slot with 4 blocks per SM; large-class blocks in
  * proportion to its share of the work; lanes of the handle; 5 sd).  Explicit
- * lanes run the tile kernel; a lockstep plan keeps its kernel otherwise and
- * reports the tiles' lanes.  No
+ * lanes run the tile kernel.  An ensemble whose default is the lockstep kernel
+ * runs it again with lanes <= 0 (in slots of small_slot strands, or, with
+ * small_slot <= 0 too, in its default plan) and reports the tiles' lanes.  No
  * counterpart in the reference (one thread per chain, ensemble_kernel.cu). */
 int dsm_set_schedule(dsm_sim* sim, int32_t small_slot, int32_t large_grid, int32_t lanes, float z_margin_sd);
 /* Current schedule: n_classes (0 = one launch over all chains), then per
@@ -247,8 +248,10 @@ int dsm_get_class_form(const dsm_sim* sim, int32_t* form);
  * the best 32-lane one), since trial windows resolve tile widths only
  * coarsely.  The ensemble advances by
  * candidates x window; its trajectory is the one it would have had without
- * the autotuner.  best (may be NULL) receives {small_slot, large_grid, lanes,
- * candidates}; best_ms the winner's kernel time.  No counterpart in the
+ * the autotuner.  An ensemble whose default is the lockstep kernel tries that
+ * plan first, and tiles must beat it by 3 %.  best (may be NULL) receives
+ * {small_slot, large_grid, lanes, candidates}, the first three as
+ * dsm_set_schedule takes them ({0, 0, 0}: the default lockstep plan); best_ms the winner's kernel time.  No counterpart in the
  * reference (fixed launch shapes). */
 int dsm_autotune(dsm_sim* sim, double window, int32_t* best, float* best_ms);
 

@@ -149,3 +149,48 @@ def test_abort_between_two_slices(dsm_mod):
     # a sum cut in two FP32 compensated pieces where the abort fell
     assert np.abs(ga - gb).max() <= 2.0**-22 * np.abs(gb).max()
     assert_bitexact(gpu_state(a), gpu_state(b), what="abort between slices")
+
+
+def plan(e):
+    k = e.step_kernel()
+    return k["lockstep"], k["lanes"], k["slot"], [(c["slot"], c["lanes"], c["grid"]) for c in e.schedule()]
+
+
+@pytest.mark.parametrize("kw", [dict(gt(64, 8, nk=200), n_chains=N), dict(nk=300, n_chains=N), dict(gt(64, 8, **SLICED))],
+                         ids=str)
+def test_autotune(dsm_mod, kw):
+    """The tuner tries the lockstep default and the tiles, keeps the default unless tiles
+    are clearly faster (they are not here), changes no trajectory, and returns what
+    set_schedule takes to make the same plan."""
+    a, b = dsm_mod.Ensemble(seed=85, **kw), dsm_mod.Ensemble(seed=85, lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    start = plan(a)
+    best = a.autotune(20.0)
+    assert best["candidates"] > 2
+    assert plan(a) == start
+    for k in range(best["candidates"]):
+        b.advance(20.0 * (k + 1))
+    assert_bitexact(gpu_state(a), gpu_state(b), what="after autotune")
+    a.set_schedule(small_slot=90 if kw["nk"] == 200 else 0, lanes=16)
+    assert not a.step_kernel()["lockstep"]
+    a.set_schedule(best["small_slot"], best["large_grid"], best["lanes"])
+    assert plan(a) == start
+    same_run(a, b, [20.0 * (best["candidates"] + 1)], "the tuner's choice again")
+
+
+@pytest.mark.parametrize("kw", [dict(gt(64, 8, nk=200), n_chains=N), dict(nk=200, n_chains=N), dict(gt(64, 8, nk=100), n_chains=1500),
+                                dict(nk=200, n_chains=1500)], ids=str)
+def test_class_form_of_a_default_plan(dsm_mod, kw):
+    """The carved form of lockstep and of small ensembles: the classes of their 16-lane
+    tiles in one launch, and the default plan back."""
+    a, b = dsm_mod.Ensemble(seed=86, **kw), dsm_mod.Ensemble(seed=86, lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    start = plan(a)
+    a.set_class_form(1)
+    assert a.class_form() == 1 and not a.step_kernel()["lockstep"] and a.schedule()[0]["lanes"] == 16
+    same_run(a, b, [20.0], "carved")
+    a.set_class_form(0)
+    assert a.class_form() == 0 and plan(a) == start
+    same_run(a, b, [40.0], "back")
