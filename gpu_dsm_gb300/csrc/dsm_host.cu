@@ -203,26 +203,42 @@ int dsm::sim_create(const dsm_params* p, bool shared, dsm_sim** out) {
 extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_create(p, false, out); }
 
 // Monodisperse equilibrium ensembles that run in the lockstep kernel
-// (dsm_lockstep.cu) rather than in tiles of 16 lanes.  It pays where most events
-// are slides, which it does four lanes to a chain, eight chains to a warp; the
-// creations and destructions, a larger share the shorter the chains and their
-// strands (small beta), go through service warps one chain at a time.  Measured
-// (events/s, lockstep against tiles; p = 64, m = 8 where G(t)):
-//   beta 1    N_K  75 2.43e9 / 2.70e9   N_K 100 2.94e9 / 2.75e9   N_K 200 3.53e9 / 2.57e9
-//     G(t)    N_K 100 1.89e9 / 2.55e9   N_K 130 2.35e9 / 2.27e9   N_K 200 2.86e9 / 2.27e9
-//     MSD     N_K 130 2.09e9 / 2.19e9   N_K 150 2.21e9 / 2.23e9   N_K 200 2.64e9 / 2.20e9
-//   beta 0.5  N_K 100 2.00e9 / 2.55e9   N_K 150 2.52e9 / 2.35e9
-//     G(t)    N_K 150 2.00e9 / 2.17e9   N_K 200 1.95e9 / 1.89e9   N_K 463 1.96e9 / 1.04e9
-//   beta 2    N_K 100 3.35e9 / 2.84e9   N_K 300 3.20e9 / 2.33e9
-//     G(t)    N_K 100 2.01e9 / 2.56e9   N_K 150 2.52e9 / 2.60e9   N_K 200 3.01e9 / 2.29e9
-// (default_schedule adds: more chains than the tiles hold at once.)  Not in the
-// server, whose memory budget does not count the kernel's buffers.  Strand
+// (dsm_lockstep.cu) rather than in tiles, and the N_K from which they do (0: not at
+// this beta).  It pays where most events are slides, which it does four lanes to a
+// chain, eight chains to a warp; creations and destructions, a larger share the
+// shorter the chains and their strands, and the samples go through service warps
+// one chain at a time.  Time in tiles over time in lockstep, 40000 chains, 800
+// events each (p = 64, m = 8 where G(t) or MSD):
+//   none  beta 0.5  N_K 170 1.03, 200 1.07, 240 1.22, 300 1.47
+//         beta 1    N_K 75 1.01, 87 1.10, 100 1.20, 120 1.07, 150 1.29, 200 1.28, 300 1.43
+//         beta 2    N_K 75 1.17, 100 1.24, 150 1.17, 200 1.37
+//         beta 4    N_K 75 1.12, 100 1.17, 200 1.29, 300 1.18
+//   G(t)  beta 0.5  N_K 150 0.90, 200 0.95, 240 1.12, 300 1.20
+//         beta 1    N_K 100 0.74, 135 0.95, 150 1.05, 175 1.12, 200 1.08, 300 1.31
+//         beta 2    N_K 130 0.86, 150 0.89, 175 1.07, 250 1.20
+//         beta 4    N_K 150 0.75, 200 0.82, 300 1.02
+//   MSD   beta 0.4  N_K 230 0.98 (6000 chains, 1600 events 1.06), 300 1.06
+//         beta 0.5  N_K 200 0.88, 240 1.05, 300 1.12
+//         beta 1    N_K 135 0.86, 150 0.95, 175 1.02, 200 1.03, 300 1.24
+//         beta 2    N_K 150 0.88, 175 1.03, 250 1.16
+//         beta 4    N_K 200 0.84, 300 1.02
+// At beta = 10 it is no faster up to the largest N_K measured, 500 (none 0.92 to
+// 1.03, G(t) 0.41 to 0.66), and slower at beta = 0.25 with a correlator (0.64 to 0.94,
+// N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)  Not
+// in the server, whose memory budget does not count the kernel's buffers.  Strand
 // sizes and the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
+static double lock_least_nk(const dsm_sim* s) {
+  const double b = (double)s->P.beta;
+  if (b > 4.0) return 0.0;
+  if (!s->corr) return std::max(75.0, 85.0 / b);
+  if (b < 0.4) return 0.0;
+  return std::max({s->ck == 2 || b > 1.0 ? 175.0 : 150.0, 75.0 * b, std::min(230.0, 120.0 / b)});
+}
 static bool prefer_lock(const dsm_sim* s) {
   const dsm_params& P = s->P;
   if (P.lanes_per_chain != 0 || s->flow || s->poly || s->shared || !s->lock_fits || s->nkmax >= 16384) return false;
-  const double f = (2.0 + 1.0 / (double)P.beta) / 3.0;
-  return (double)P.nk >= (s->corr ? 150.0 * std::max(1.0, f) : 100.0 * f);
+  const double least = lock_least_nk(s);
+  return least > 0.0 && (double)P.nk >= least;
 }
 
 int dsm::sim_setup(dsm_sim* s) {

@@ -1241,7 +1241,7 @@ struct LockShape {
   int lanes, sb;
 };
 static LockShape lock_shape(int slot_cap) {
-  for (int sb : {2, 3, 5, 9})
+  for (int sb : {3, 5, 9})
     if (slot_cap <= 16 * sb) return {4, sb};
   for (int sb : {8, 12})
     if (slot_cap <= 32 * sb) return {8, sb};
@@ -1257,7 +1257,6 @@ size_t lock_block_bytes(int slot_cap, int tiles) {
 template <int CK, int MB>
 static void* lock_pick(const LockShape& f) {
   switch (f.sb) {
-    case 2: return (void*)k_lock<CK, 4, 2, 128, MB>;
     case 3: return (void*)k_lock<CK, 4, 3, 128, MB>;
     case 5: return (void*)k_lock<CK, 4, 5, 128, MB>;
     case 9: return (void*)k_lock<CK, 4, 9, 128, MB>;
