@@ -224,9 +224,11 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_
 //         beta 4    N_K 200 0.84, 300 1.02
 // At beta = 10 it is no faster up to the largest N_K measured, 500 (none 0.92 to
 // 1.03, G(t) 0.41 to 0.66), and slower at beta = 0.25 with a correlator (0.64 to 0.94,
-// N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)  Not
-// in the server, whose memory budget does not count the kernel's buffers.  Strand
-// sizes and the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
+// N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)
+// Not with a GEX background, whose partner law every creation would evaluate in a
+// service warp (N_K = 100 and 200, with and without G(t): 0.44 to 0.50).  Not in the
+// server, whose memory budget does not count the kernel's buffers.  Strand sizes and
+// the split of a strand work in 16 and 64 bits there, hence N_K < 2^14.
 static double lock_least_nk(const dsm_sim* s) {
   const double b = (double)s->P.beta;
   if (b > 4.0) return 0.0;
@@ -236,7 +238,8 @@ static double lock_least_nk(const dsm_sim* s) {
 }
 static bool prefer_lock(const dsm_sim* s) {
   const dsm_params& P = s->P;
-  if (P.lanes_per_chain != 0 || s->flow || s->poly || s->shared || !s->lock_fits || s->nkmax >= 16384) return false;
+  if (P.lanes_per_chain != 0 || s->flow || s->poly || P.pd_flag != 0 || s->shared || !s->lock_fits || s->nkmax >= 16384)
+    return false;
   const double least = lock_least_nk(s);
   return least > 0.0 && (double)P.nk >= least;
 }

@@ -510,21 +510,24 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
     const float4 qo = Q[ia];
     // even lanes the event's own words, odd lanes the creation's
     const U4 w = lock_words(E, (lane & 1) ? P_CREATE : P_EVENT, step, c);
-    const uint32_t w2 = wshfl(w.z, 0), w3 = wshfl(w.w, 0);
+    const uint32_t w2 = wshfl(w.z, 0);
     // lanes 0 and 1 a pair of normal deviates each, lane 2 the lifetime's power
     const uint32_t gx = wshfl(w.x, 1), gy = wshfl(w.y, 1), gz = wshfl(w.z, 1), gw = wshfl(w.w, 1);
-    const PcdDev pp = partner_pcd(E, w3, cdc);
+    // (one N_K, no GEX background: the ensemble's own partner law)
+    const PcdDev& pp = E.pcd;
+    const float pA = cdc ? pp.Adt_ : pp.At_, pD = cdc ? pp.Ddt_ : pp.Dt_, pC = cdc ? pp.Cdt_ : pp.Ct_;
+    const float pB = cdc ? pp.Bdt_ : pp.one_minus_g;
     const float u = u01(w2);
-    const float base = cdc ? __fmaf_rn(u, pp.Adt_, pp.Ddt_) : __fmaf_rn(u, pp.At_, pp.Dt_);
+    const float base = __fmaf_rn(u, pA, pD);
     const float lg = m_log(lane == 0 ? u01(gx) : lane == 1 ? u01(gz) : base);
     float sn, cs;
     m_sincos2pi((lane == 0 ? gy : gw) >> 8, &sn, &cs);
     // (other lanes' logarithms may be positive, a slow case of the square root)
     const float rr = __fsqrt_rn(lane < 2 ? __fmul_rn(-2.0f, lg) : 1.0f);
     const float ga = __fmul_rn(rr, cs), gb = __fmul_rn(rr, sn);
-    const float pw = wshfl(m_exp(__fmul_rn(cdc ? pp.Cdt_ : pp.Ct_, lg)), 2);
+    const float pw = wshfl(m_exp(__fmul_rn(pC, lg)), 2);
     const float g0 = wshfl(ga, 0), g1 = wshfl(gb, 0), g2 = wshfl(ga, 1);
-    trate = cd ? ((u < (cdc ? pp.Bdt_ : pp.one_minus_g)) ? pw : pp.tau_d_inv) : 0.0f;
+    trate = cd ? ((u < pB) ? pw : pp.tau_d_inv) : 0.0f;
     int newn = 0;
     if (cdc) {
       newn = lock_split(rem, wsel, N1) + 1;

@@ -28,14 +28,14 @@ def same_run(a, b, times, what):
 @pytest.mark.parametrize("kw,lanes", [
     (dict(nk=75, beta=4.0), 4), (dict(nk=90, beta=3.0), 4), (dict(nk=100), 4), (dict(nk=131), 4),
     (dict(nk=200, beta=0.5), 8), (dict(nk=463, beta=0.5), 8), (dict(nk=100, cd_flag=0), 4), (dict(nk=100, z_max=52), 4),
-    (dict(nk=100, gex=(1.0, 1.0, 1000.0, 100.0)), 4), (gt(16, 2, nk=151), 4), (gt(64, 8, nk=200), 4),
+    (gt(16, 2, nk=151), 4), (gt(64, 8, nk=200), 4),
     (gt(96, 4, nk=240, beta=0.5), 8), (dict(gt(8, 2, nk=175), eq_type=2), 4), (dict(gt(8, 2, nk=300), eq_type=2), 8)], ids=str)
 def test_kernel_of_the_plan(dsm_mod, kw, lanes):
     k = dsm_mod.Ensemble(n_chains=N, seed=71, **kw).step_kernel()
     assert k["lockstep"] and k["lanes"] == lanes
 
 
-@pytest.mark.parametrize("kw", [dict(nk=20), dict(nk=500, beta=10.0), gt(64, 8, nk=200, beta=0.5), gt(64, 8, nk=150, beta=2.0),
+@pytest.mark.parametrize("kw", [dict(nk=20), dict(nk=200, gex=(1.0, 1.0, 1000.0, 100.0)), dict(nk=500, beta=10.0), gt(64, 8, nk=200, beta=0.5), gt(64, 8, nk=150, beta=2.0),
                                 gt(64, 8, nk=200, beta=4.0), dict(gt(64, 8, nk=150), eq_type=2), gt(64, 8, nk=300, beta=0.25),
                                 dict(nk=200, lanes_per_chain=16), dict(nk=200, lanes_per_chain=32),
                                 dict(nk=200, kappa=(0.0, 2.0e-3) + (0.0,) * 7)], ids=str)
