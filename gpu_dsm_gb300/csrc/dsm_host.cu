@@ -202,6 +202,8 @@ int dsm::sim_create(const dsm_params* p, bool shared, dsm_sim** out) {
 
 extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_create(p, false, out); }
 
+constexpr double kEventsPerTau = 0.21;  // of a chain, per Kuhn step (a little more for small beta)
+
 // Monodisperse equilibrium ensembles that run in the lockstep kernel
 // (dsm_lockstep.cu) rather than in tiles, and the N_K from which they do (0: not at
 // this beta).  It pays where most events are slides, which it does four lanes to a
@@ -225,6 +227,16 @@ extern "C" int dsm_create(const dsm_params* p, dsm_sim** out) { return dsm::sim_
 // At beta = 10 it is no faster up to the largest N_K measured, 500 (none 0.92 to
 // 1.03, G(t) 0.41 to 0.66), and slower at beta = 0.25 with a correlator (0.64 to 0.94,
 // N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)
+// These samples are a tau apart (kEventsPerTau N_K events).  Each costs a service warp
+// more than it does a tile, so samples that are few events apart move the line, the
+// less the longer the chains (time in tiles over lockstep, 16384 chains, 800 events,
+// at the events between two samples):
+//   G(t)  N_K 200 (beta 1)    42 1.19, 21 1.11, 10 0.93, 4 0.63
+//         N_K 300 (beta 1)    63 1.29, 31 1.20, 16 1.09, 6 0.86
+//         N_K 463 (beta 0.5)  97 1.72, 24 1.50, 10 1.28, 5 1.08
+//   MSD   N_K 200 (beta 1)    42 1.13, 21 1.02, 10 0.79
+//         N_K 300 (beta 1)    63 1.23, 31 1.12, 16 0.99, 6 0.69
+//         N_K 463 (beta 0.5)  97 1.62, 24 1.37, 10 1.10, 5 0.81
 // Not with a GEX background, whose partner law every creation would evaluate in a
 // service warp (N_K = 100 and 200, with and without G(t): 0.44 to 0.50).  Not in the
 // server, whose memory budget does not count the kernel's buffers.  Strand sizes and
@@ -240,8 +252,9 @@ static bool prefer_lock(const dsm_sim* s) {
   const dsm_params& P = s->P;
   if (P.lanes_per_chain != 0 || s->flow || s->poly || P.pd_flag != 0 || s->shared || !s->lock_fits || s->nkmax >= 16384)
     return false;
-  const double least = lock_least_nk(s);
-  return least > 0.0 && (double)P.nk >= least;
+  const double least = lock_least_nk(s), x = (double)P.nk / std::max(1.0, least);
+  if (least == 0.0 || x < 1.0) return false;
+  return !s->corr || kEventsPerTau * (double)P.nk * P.sync_dt >= (s->ck == 2 ? 36.0 : 30.0) / std::pow(x, 1.7);
 }
 
 int dsm::sim_setup(dsm_sim* s) {
@@ -521,7 +534,7 @@ static int plan_buffers(dsm_sim* s) {
 // 500 events per chain; none under an event limit (it counts events, not time)
 static int launch_slices(const dsm_sim* s, double dt_tau, int64_t step_limit) {
   if (s->sub_max <= 1 || step_limit >= 0) return 1;
-  const double ev = 0.21 * (double)s->P.nk * std::max(0.0, dt_tau);
+  const double ev = kEventsPerTau * (double)s->P.nk * std::max(0.0, dt_tau);
   return std::max(1, std::min(s->sub_max, (int)std::min(ev / 500.0, 1000.0)));
 }
 

@@ -16,7 +16,7 @@ SLICED = dict(nk=300, beta=0.5, n_chains=6000)
 
 
 def gt(p, m, **kw):
-    return dict(eq_type=1, corr_p=p, corr_m=m, sync_dt=0.25, t_end=4000.0, **kw)
+    return dict(dict(eq_type=1, corr_p=p, corr_m=m, sync_dt=1.0, t_end=4000.0), **kw)
 
 
 def same_run(a, b, times, what):
@@ -29,19 +29,41 @@ def same_run(a, b, times, what):
     (dict(nk=75, beta=4.0), 4), (dict(nk=90, beta=3.0), 4), (dict(nk=100), 4), (dict(nk=131), 4),
     (dict(nk=200, beta=0.5), 8), (dict(nk=463, beta=0.5), 8), (dict(nk=100, cd_flag=0), 4), (dict(nk=100, z_max=52), 4),
     (gt(16, 2, nk=151), 4), (gt(64, 8, nk=200), 4),
-    (gt(96, 4, nk=240, beta=0.5), 8), (dict(gt(8, 2, nk=175), eq_type=2), 4), (dict(gt(8, 2, nk=300), eq_type=2), 8)], ids=str)
+    (gt(96, 4, nk=240, beta=0.5), 8), (gt(8, 2, nk=175, eq_type=2), 4),
+    (gt(64, 8, nk=300, sync_dt=0.25), 8), (gt(64, 8, nk=463, beta=0.5, sync_dt=0.1), 8), (gt(8, 2, nk=300, sync_dt=0.5, eq_type=2), 8)], ids=str)
 def test_kernel_of_the_plan(dsm_mod, kw, lanes):
     k = dsm_mod.Ensemble(n_chains=N, seed=71, **kw).step_kernel()
     assert k["lockstep"] and k["lanes"] == lanes
 
 
 @pytest.mark.parametrize("kw", [dict(nk=20), dict(nk=200, gex=(1.0, 1.0, 1000.0, 100.0)), dict(nk=500, beta=10.0), gt(64, 8, nk=200, beta=0.5), gt(64, 8, nk=150, beta=2.0),
-                                gt(64, 8, nk=200, beta=4.0), dict(gt(64, 8, nk=150), eq_type=2), gt(64, 8, nk=300, beta=0.25),
+                                gt(64, 8, nk=200, beta=4.0), gt(64, 8, nk=150, eq_type=2), gt(64, 8, nk=300, beta=0.25),
+                                gt(64, 8, nk=200, sync_dt=0.25), gt(64, 8, nk=200, sync_dt=0.5, eq_type=2),
                                 dict(nk=200, lanes_per_chain=16), dict(nk=200, lanes_per_chain=32),
                                 dict(nk=200, kappa=(0.0, 2.0e-3) + (0.0,) * 7)], ids=str)
 def test_tiles_otherwise(dsm_mod, kw):
     assert not dsm_mod.Ensemble(n_chains=N, seed=71, **kw).step_kernel()["lockstep"]
     assert not dsm_mod.Ensemble(n_chains=900, nk=200, seed=71).step_kernel()["lockstep"]
+
+
+@pytest.mark.parametrize("kw", [gt(16, 2, nk=300, sync_dt=0.25), gt(64, 8, nk=200), gt(96, 4, nk=240, beta=0.5),
+                                gt(64, 8, nk=300, sync_dt=0.5, eq_type=2), gt(8, 2, nk=175, eq_type=2)], ids=str)
+def test_correlators(dsm_mod, kw):
+    """G(t) and MSD sums of lockstep plans against 16-lane tiles, over windows that end
+    inside, at and after full sample buffers (64 samples)."""
+    a, b = dsm_mod.Ensemble(n_chains=N, seed=80, **kw), dsm_mod.Ensemble(n_chains=N, seed=80, lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    dt = kw["sync_dt"]
+    for samples in (80, 95, 159, 192):
+        t = samples * dt
+        assert a.advance(t) == b.advance(t)
+        assert a.step_kernel()["lockstep"]
+        ga, ca = a.gt_raw()
+        gb, cb = b.gt_raw()
+        assert np.array_equal(ca, cb) and np.array_equal(ga, gb)
+    assert_bitexact(gpu_state(a), gpu_state(b), what="correlator")
+    assert np.array_equal(a.r1(), b.r1())
 
 
 def test_slices_of_a_launch(dsm_mod):
