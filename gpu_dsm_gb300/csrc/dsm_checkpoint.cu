@@ -191,5 +191,6 @@ extern "C" int dsm_checkpoint_load(dsm_sim* s, const char* path) {
   s->t_done = h.t_done;
   s->t_window = h.t_done;
   s->events_total = h.events_total;
+  s->events_base = 0;
   return DSM_OK;
 }

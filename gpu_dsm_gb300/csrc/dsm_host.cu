@@ -257,6 +257,28 @@ static bool prefer_lock(const dsm_sim* s) {
   return !s->corr || kEventsPerTau * (double)P.nk * P.sync_dt >= (s->ck == 2 ? 36.0 : 30.0) / std::pow(x, 1.7);
 }
 
+// Events per chain from which a launch is faster in the lockstep kernel.  It brings a
+// chain in and out at several times the cost of a tile (a service warp does it, two
+// for up to 16 slots; the vectors go back to strand order) and has to earn that by
+// its events.  Measured crossings, 8192 to 65536 chains (more chains, later):
+//   none  beta 1    N_K 87 230 to 380, 100 160 to 220, 150 100 to 170, 200 60 to 150, 300 95
+//         beta 0.5  N_K 170 380 to 600, 240 190, 463 80   beta 2  N_K 75 280, 150 170 to 320, 300 100
+//         beta 4    N_K 75 390 to 750, 150 290 to 450, 300 340
+//   G(t)  beta 1    N_K 150 260 to 600, 200 180 to 500, 300 130 to 180
+//         beta 0.5  N_K 240 340 to 380, 300 160 to 240, 463 25 to 35 (8 tiles per SM)
+//         beta 2    N_K 175 390 to 550, 300 105 to 130   beta 4  N_K 300 500 to 700
+//   MSD   beta 1    N_K 175 600, 200 210 to 700, 300 140 to 200, which with tiles of
+//         16 lanes where 32 are faster is 50
+// Below them the start of a window counts: 0.1 tau of 16384 chains of N_K = 200, G(t),
+// 0.15 ms in tiles and 0.34 in lockstep, 1 tau 0.47 and 0.68, 5 tau 1.78 and 1.73.
+static double lock_least_events(const dsm_sim* s, int tile_lanes, int tiles_per_sm) {
+  const double x = (double)s->P.nk / lock_least_nk(s);
+  if (!s->corr) return std::max(100.0, 350.0 * std::max(1.0, 0.5 * (double)s->P.beta) / x);
+  if (s->ck == 2 && tile_lanes != 16) return 50.0;
+  const double r = std::min(1.0, tiles_per_sm / 16.0);
+  return std::max(30.0, 600.0 * r * r / (x * x));
+}
+
 int dsm::sim_setup(dsm_sim* s) {
   dsm_params& P = s->P;
   if (P.nk < 1 || P.n_chains < 1 || !(P.beta > 0.0f)) return fail(s, DSM_ERR_INVALID, "invalid nk / n_chains / beta");
@@ -541,6 +563,7 @@ static int launch_slices(const dsm_sim* s, double dt_tau, int64_t step_limit) {
 // One launch over all chains with slots of the full capacity
 static int plan_single(dsm_sim* s) {
   s->classes.clear();
+  s->lock_events = 0.0;
   ++s->sched_version;
   s->cfg.slot_cap = s->cap;
   int smem_optin = 0;
@@ -560,6 +583,7 @@ static int plan_single(dsm_sim* s) {
 
 int dsm::plan_classes(dsm_sim* s, int small_cap, int big_grid, int lanes, float margin_sd) {
   s->classes.clear();
+  s->lock_events = 0.0;
   s->carved = false;
   s->margin_sd = margin_sd;
   ++s->sched_version;
@@ -834,9 +858,40 @@ static int default_schedule(dsm_sim* s) {
   const double zb = 1.0 + (nk - 1.0) * pe + 5.0 * std::sqrt(std::max(0.0, (nk - 1.0) * pe * (1.0 - pe))) + 2.0;
   const int slot = std::max(8, (int)std::ceil(zb));
   if (lock_lanes(std::min(slot, s->cap)) == 0) return rc;
+  // the tiles stay as the second plan, for short windows (choose_plan)
+  const double least = lock_least_events(s, t.lanes, s->blocks_per_sm * step_tiles(s->flow, t));
+  // (MSD: with 16 lanes, whose order of the centre-of-mass sums is the lockstep kernel's)
+  bool two = true;
+  if (s->ck == 2 && t.lanes != 16) {
+    s->cfg.lanes = 16;
+    two = plan_single(s) == DSM_OK;
+  }
+  s->other = StepPlan{s->cfg, s->classes, s->cleanup, s->grid, s->blocks_per_sm, s->sub_max};
   s->cfg.lanes = 16;
   s->cfg.lock = s->lock_default = true;
-  return slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
+  const int rl = slot >= s->cap ? plan_single(s) : plan_classes(s, slot, 0, 16, 0.f);
+  if (rl == DSM_OK && two) s->lock_events = least;
+  return rl;
+}
+
+// The plan of a launch of windows of dt_tau (or up to step_limit events per chain):
+// a default lockstep ensemble runs tiles where the chains do fewer than lock_events
+// events.  The sums and the state are the same.
+static void choose_plan(dsm_sim* s, double dt_tau, int64_t step_limit) {
+  if (s->lock_events <= 0.0) return;
+  double ev = kEventsPerTau * (double)s->P.nk * std::max(0.0, dt_tau);
+  if (step_limit >= 0) {
+    // (after an event-limited launch the chains are behind the handle's time)
+    const double left = (double)step_limit - (double)(s->events_total - s->events_base) / (double)s->P.n_chains;
+    ev = dt_tau > 0.0 ? std::min(ev, left) : left;
+  }
+  if ((ev >= s->lock_events) == s->cfg.lock) return;
+  std::swap(s->cfg, s->other.cfg);
+  s->classes.swap(s->other.classes);
+  std::swap(s->cleanup, s->other.cleanup);
+  std::swap(s->grid, s->other.grid);
+  std::swap(s->blocks_per_sm, s->other.blocks_per_sm);
+  std::swap(s->sub_max, s->other.sub_max);
 }
 
 // Blocks per SM of one launch with one chain per warp and full-capacity slots,
@@ -1114,6 +1169,7 @@ extern "C" int dsm_init_equilibrium(dsm_sim* s) {
   CK(launch_init(s->d_ens, s->h, s->cap, s->st));
   CK(cudaStreamSynchronize(s->st));
   s->lost = false;
+  s->events_base = s->events_total;
   return DSM_OK;
 }
 
@@ -1166,6 +1222,7 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
   s->lost = false;
+  s->events_base = s->events_total;
   return DSM_OK;
 }
 
@@ -1324,6 +1381,7 @@ int dsm::sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit) {
   EnsDev& E = s->h;
   E.t_end_ticks = (int64_t)std::llrint(t_end * TICKS);
   s->t_window = t_end;
+  choose_plan(s, t_end - s->t_done, step_limit);
   E.step_limit = step_limit < 0 ? INT64_MAX : step_limit;
   E.watchdog_events = window_watchdog(s, t_end - s->t_done);
   E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
@@ -1438,12 +1496,13 @@ static int series_prepare(dsm_sim* s, int n, cudaGraphExec_t* exec) {
     s->ser_version = s->sched_version;
   }
   if (!exec) return DSM_OK;  // buffers only (windows issued directly)
+  const int key = 2 * n + (s->cfg.lock ? 1 : 0);  // (choose_plan does not change the schedule's version)
   for (auto& g : s->ser_graphs)
-    if (g.first == n) { *exec = g.second; return DSM_OK; }
+    if (g.first == key) { *exec = g.second; return DSM_OK; }
   cudaGraphExec_t e = nullptr;
   const int rc = series_capture(s, n, &e);
   if (rc != DSM_OK) return rc;
-  s->ser_graphs.push_back({n, e});
+  s->ser_graphs.push_back({key, e});
   *exec = e;
   return DSM_OK;
 }
@@ -1461,6 +1520,7 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   // 10-20 % slower on the 262144-chain log-normal melt (a graph of one window
   // did not), while a few launches per window cost nothing next to windows of
   // seconds.
+  choose_plan(s, (ends[n - 1] - s->t_done) / n, -1);
   const bool direct = !s->classes.empty();
   cudaGraphExec_t exec = nullptr;
   int rc = series_prepare(s, n, direct ? nullptr : &exec);
@@ -1850,6 +1910,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   auto cap_class = [](int cap) { int c = 16; while (c < cap) c <<= 1; return c; };
   std::vector<Group> groups;
   for (int i = 0; i < n; ++i) {
+    choose_plan(sims[i], t_end[i] - sims[i]->t_done, step_limit ? step_limit[i] : -1);
     const bool fl = sims[i]->flow;
     const int co = sims[i]->ck;
     const int cc = cap_class(sims[i]->cap), cp = co ? sims[i]->cp : 0;

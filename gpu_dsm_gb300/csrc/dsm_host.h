@@ -69,6 +69,13 @@ struct SizeClass {
   int grid = 0, bps = 0;
   int stream = 0;  // 0 the handle's stream, 1 side, 2 side2, 3 side3
 };
+// A launch plan that is not the current one (choose_plan)
+struct StepPlan {
+  LaunchCfg cfg{4, 0, 0, 32};
+  std::vector<SizeClass> classes;
+  SizeClass cleanup;
+  int grid = 0, blocks_per_sm = 0, sub_max = 1;
+};
 }  // namespace dsm
 
 struct dsm_sim {
@@ -142,6 +149,11 @@ struct dsm_sim {
   bool shared = false;     // runs next to other ensembles on the device (dsm_server)
   bool lock_fits = false;  // device memory for the lockstep kernel's buffers
   bool lock_default = false;  // the lockstep kernel is this ensemble's default (default_schedule)
+  // a default lockstep plan has tiles beside it for launches of fewer events per
+  // chain than lock_events (0: one plan); choose_plan swaps the two
+  double lock_events = 0.0;
+  dsm::StepPlan other;
+  uint64_t events_base = 0;  // events_total when the chains were set
   bool by_default = false;    // monodisperse: the plan is the default one, not one that was asked for
   // one chain per warp because all chains are resident so (small_schedule): the
   // slot of the two-per-warp plan, which a batch of such ensembles may need; else 0

@@ -222,7 +222,9 @@ int dsm_set_schedule(dsm_sim* sim, int32_t small_slot, int32_t large_grid, int32
 int dsm_get_schedule(const dsm_sim* sim, int32_t* n_classes, int32_t* info);
 
 /* Step kernel of the plan's last (or only) class: info = {1 lockstep or 0 tiles,
- * lanes per chain, slot strands, time slices of the last launch}. */
+ * lanes per chain, slot strands, time slices of the last launch}.  An ensemble whose
+ * default is the lockstep kernel runs tiles in launches of few events per chain;
+ * this and dsm_get_schedule report the plan of the last launch. */
 int dsm_get_step_kernel(const dsm_sim* sim, int32_t info[4]);
 
 /* How size classes launch (equilibrium ensembles whose small class runs 16

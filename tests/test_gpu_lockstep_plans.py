@@ -55,7 +55,7 @@ def test_correlators(dsm_mod, kw):
     for x in (a, b):
         x.init_equilibrium()
     dt = kw["sync_dt"]
-    for samples in (80, 95, 159, 192):
+    for samples in (80, 100, 160, 192):
         t = samples * dt
         assert a.advance(t) == b.advance(t)
         assert a.step_kernel()["lockstep"]
@@ -66,13 +66,72 @@ def test_correlators(dsm_mod, kw):
     assert np.array_equal(a.r1(), b.r1())
 
 
+@pytest.mark.parametrize("kw", [dict(nk=131), dict(nk=200, beta=0.5), dict(nk=463, beta=0.5), dict(nk=90, beta=3.0),
+                                dict(nk=100, cd_flag=0), dict(nk=100, z_max=52)], ids=str)
+def test_against_the_oracle(dsm_mod, oracle_mod, kw):
+    g, o = dsm_mod.Ensemble(n_chains=N, seed=87, **kw), oracle_mod.Oracle(n_chains=N, seed=87, **kw)
+    g.init_equilibrium()
+    o.init_equilibrium()
+    assert g.advance(30.0) == o.run(30.0)
+    assert g.step_kernel()["lockstep"]
+    assert_bitexact(gpu_state(g), o.get_state(), what=f"{kw}")
+
+
+@pytest.mark.parametrize("q", [12.0, 15.0, 17.0, 40.0])
+def test_exponents_beyond_the_short_form(dsm_mod, oracle_mod, q):
+    """Strands so long that sliding exponents pass the limit of the short exponential."""
+    kw = dict(nk=200, n_chains=N, seed=88, beta=0.5)
+    g, o = dsm_mod.Ensemble(**kw), oracle_mod.Oracle(**kw)
+    g.init_equilibrium()
+    heads, qn, tau = g.get_chains()
+    rng = np.random.default_rng(5)
+    for c in rng.choice(N, N // 4, replace=False):
+        qn[c, int(rng.integers(2, int(heads["Z"][c]) - 2)), :3] = np.float32(q) * np.array([0.6, 0.0, 0.8], np.float32)
+    g.set_chains(heads, qn, tau)
+    o.set_state(heads["Z"], qn, tau, T=g.get_ext()["T"])
+    assert g.advance(20.0) == o.run(20.0)
+    assert g.step_kernel()["lockstep"]
+    assert_bitexact(gpu_state(g), o.get_state(), what=f"|Q|={q}")
+
+
+@pytest.mark.parametrize("kw", [dict(nk=100), gt(64, 8, nk=200), gt(64, 8, nk=200, eq_type=2), gt(64, 8, **SLICED),
+                                dict(gt(16, 2, eq_type=2), **SLICED), dict(nk=100, z_max=52)], ids=str)
+def test_short_and_long_windows(dsm_mod, kw):
+    """A default lockstep ensemble runs tiles where a launch has few events per chain; the
+    state, and what does not depend on where the windows end, are those of tiles."""
+    kw = dict(dict(n_chains=N), **kw)
+    a, b = dsm_mod.Ensemble(seed=89, **kw), dsm_mod.Ensemble(seed=89, lanes_per_chain=16, **kw)
+    for x in (a, b):
+        x.init_equilibrium()
+    t = 0.0
+    for dt, lock in ((0.25, False), (30.0, True), (0.5, False), (0.7, False), (40.0, True)):
+        t += dt
+        assert a.advance(t) == b.advance(t)
+        assert a.step_kernel()["lockstep"] == lock
+    for dt, n, lock in ((0.5, 4, False), (20.0, 2, True), (0.5, 4, False)):
+        assert a.advance_series(dt, n)[0] == b.advance_series(dt, n)[0]
+        assert a.step_kernel()["lockstep"] == lock
+        t += dt * n
+    for dt, lock in ((0.5, False), (30.0, True)):
+        t += dt
+        assert dsm_mod.advance_batch([a], t)[0] == b.advance(t)
+        assert a.step_kernel()["lockstep"] == lock
+    done = int(b.get_ext()["step"].mean())
+    for limit, lock in ((done + 40, False), (done + 1500, True)):
+        assert a.advance(1.0e6, step_limit=limit) == b.advance(1.0e6, step_limit=limit)
+        assert a.step_kernel()["lockstep"] == lock
+    assert_bitexact(gpu_state(a), gpu_state(b), what="short and long windows")
+    if "eq_type" in kw:
+        assert np.array_equal(a.gt_raw()[0], b.gt_raw()[0]) and np.array_equal(a.gt_raw()[1], b.gt_raw()[1])
+
+
 def test_slices_of_a_launch(dsm_mod):
     e = dsm_mod.Ensemble(seed=74, **SLICED)
     e.init_equilibrium()
     e.advance(55.0)
     assert e.step_kernel() == {"lockstep": True, "lanes": 8, "slot": e.step_kernel()["slot"], "slices": 4}
-    e.advance(55.5)  # a few dozen events per chain
-    assert e.step_kernel()["slices"] == 1
+    e.advance(65.0)  # some 600 events per chain
+    assert e.step_kernel()["lockstep"] and e.step_kernel()["slices"] == 1
 
 
 @pytest.mark.parametrize("ends,slices", [((80.0, 81.0, 161.0), 1), ((80.0, 160.0, 240.0), 4)], ids=str)
@@ -100,9 +159,10 @@ def test_batch_of_lockstep_ensembles(dsm_mod):
     assert [x.step_kernel()["lockstep"] for x in a] == [True, True, True, False, False]
     for x in a + b:
         x.init_equilibrium()
-    for t in (1.5, 4.0):
+    for t in (20.0, 45.0):
         ev = dsm_mod.advance_batch(a, t)
         assert list(ev) == [x.advance(t) for x in b]
+        assert [x.step_kernel()["lockstep"] for x in a] == [True, True, True, False, False]
     for x, y in zip(a, b):
         assert_bitexact(gpu_state(x), gpu_state(y), what="batch")
     # (chains of the first outgrow the group's slot, which is the second's: their
@@ -122,7 +182,8 @@ def test_series(dsm_mod, z_max):
     for x in (a, b):
         x.init_equilibrium()
     for _ in range(2):
-        assert a.advance_series(0.5, 3)[0] == b.advance_series(0.5, 3)[0]
+        assert a.advance_series(20.0, 3)[0] == b.advance_series(20.0, 3)[0]
+        assert a.step_kernel()["lockstep"]
     assert_bitexact(gpu_state(a), gpu_state(b), what="series")
 
 
@@ -130,19 +191,20 @@ def test_saved_and_reloaded(dsm_mod, tmp_path):
     kw = dict(gt(64, 8, nk=200), n_chains=N, seed=78)
     a, b, c = dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(lanes_per_chain=16, **kw)
     a.init_equilibrium()
-    a.advance(3.0)
+    a.advance(20.0)
     a.checkpoint(str(tmp_path / "k"))
     for x in (b, c):
         x.restore(str(tmp_path / "k"))
     assert b.step_kernel()["lockstep"]
-    a.advance(8.0)
-    same_run(b, c, [8.0], "restored")
+    a.advance(45.0)
+    same_run(b, c, [45.0], "restored")
+    assert a.step_kernel()["lockstep"] and b.step_kernel()["lockstep"]
     assert_bitexact(gpu_state(a), gpu_state(b), what="continued")
     assert np.array_equal(a.gt_raw()[0], b.gt_raw()[0]) and np.array_equal(b.gt_raw()[0], c.gt_raw()[0])
     a.save(str(tmp_path / "c"))
     for x in (b, c):
         x.load(str(tmp_path / "c"))
-    same_run(b, c, [10.0], "loaded")
+    same_run(b, c, [65.0], "loaded")
 
 
 def test_abort_between_two_slices(dsm_mod):

@@ -17,7 +17,7 @@ def test_wait_that_runs_out(dsm_mod, oracle_mod, tmp_path):
     g.advance(0.5)
     g.set_wait_polls(1)  # no request is served within two polls of the launch's start
     with pytest.raises(dsm_mod.DSMError, match="ran out"):
-        g.advance(4.0)
+        g.advance(30.0)
     g.set_wait_polls(0)
     refused = [lambda: g.advance(4.0), lambda: g.advance_start(4.0), lambda: g.advance_series(1.0, 2),
                lambda: g.autotune(1.0), g.get_chains, g.get_ext, g.stress, g.gt, g.gt_raw, g.distributions, g.r1,
@@ -29,7 +29,8 @@ def test_wait_that_runs_out(dsm_mod, oracle_mod, tmp_path):
     o = oracle_mod.Oracle(corr=True, sync_dt=0.5, t_end=100.0, corr_p=16, corr_m=2, **kw)
     g.init_equilibrium()
     o.init_equilibrium()
-    assert g.advance(4.0) == o.run(4.0)
+    assert g.advance(30.0) == o.run(30.0)
+    assert g.step_kernel()["lockstep"]
     assert_bitexact(gpu_state(g), o.get_state(), what="after a lost launch")
 
 
@@ -42,12 +43,12 @@ def test_batch_keeps_the_other_groups(dsm_mod):
         x.init_equilibrium()
     a.set_wait_polls(1)
     with pytest.raises(dsm_mod.DSMError):
-        dsm_mod.advance_batch([b, a], 2.0)
+        dsm_mod.advance_batch([b, a], 20.0)
     with pytest.raises(dsm_mod.DSMError, match="set them anew"):
         a.get_chains()
-    c.advance(2.0)
+    c.advance(20.0)
     assert_bitexact(gpu_state(b), gpu_state(c), what="other group")
-    assert b.advance(3.0) == c.advance(3.0)
+    assert b.advance(21.0) == c.advance(21.0)
 
 
 def test_short_limit_with_progress(dsm_mod):
