@@ -211,10 +211,11 @@ constexpr double kEventsPerTau = 0.21;  // of a chain, per Kuhn step (a little m
 // shorter the chains and their strands, and the samples go through service warps
 // one chain at a time.  Time in tiles over time in lockstep, 40000 chains, 800
 // events each (p = 64, m = 8 where G(t) or MSD):
-//   none  beta 0.5  N_K 170 1.03, 200 1.07, 240 1.22, 300 1.47
-//         beta 1    N_K 75 1.01, 87 1.10, 100 1.20, 120 1.07, 150 1.29, 200 1.28, 300 1.43
-//         beta 2    N_K 75 1.17, 100 1.24, 150 1.17, 200 1.37
-//         beta 4    N_K 75 1.12, 100 1.17, 200 1.29, 300 1.18
+//   none  beta 0.25 N_K 150 0.88, 200 1.07, 260 1.22, 320 1.06
+//         beta 0.5  N_K 115 0.96, 130 1.12, 170 1.07, 200 1.11, 240 1.45, 300 1.51
+//         beta 1    N_K 60 0.94, 67 1.00, 75 1.07, 100 1.29, 150 1.30, 200 1.40, 300 1.71
+//         beta 2    N_K 40 0.95, 50 1.07, 60 1.18, 75 1.29, 100 1.35, 150 1.37, 200 1.41
+//         beta 4    N_K 40 0.96, 50 1.06, 60 1.15, 100 1.32, 200 1.42
 //   G(t)  beta 0.5  N_K 150 0.90, 200 0.95, 240 1.12, 300 1.20
 //         beta 1    N_K 100 0.74, 135 0.95, 150 1.05, 175 1.12, 200 1.08, 300 1.31
 //         beta 2    N_K 130 0.86, 150 0.89, 175 1.07, 250 1.20
@@ -224,9 +225,9 @@ constexpr double kEventsPerTau = 0.21;  // of a chain, per Kuhn step (a little m
 //         beta 1    N_K 135 0.86, 150 0.95, 175 1.02, 200 1.03, 300 1.24
 //         beta 2    N_K 150 0.88, 175 1.03, 250 1.16
 //         beta 4    N_K 200 0.84, 300 1.02
-// At beta = 10 it is no faster up to the largest N_K measured, 500 (none 0.92 to
-// 1.03, G(t) 0.41 to 0.66), and slower at beta = 0.25 with a correlator (0.64 to 0.94,
-// N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)
+// At beta = 10 it is no faster before some 800 events (none 0.99 to 1.12, N_K 75 to
+// 500), with G(t) not at all (0.41 to 0.66); slower at beta = 0.25 with a correlator
+// (0.64 to 0.94, N_K 150 to 320).  (default_schedule adds: more chains than the tiles hold at once.)
 // These samples are a tau apart (kEventsPerTau N_K events).  Each costs a service warp
 // more than it does a tile, so samples that are few events apart move the line, the
 // less the longer the chains (time in tiles over lockstep, 16384 chains, 800 events,
@@ -244,7 +245,7 @@ constexpr double kEventsPerTau = 0.21;  // of a chain, per Kuhn step (a little m
 static double lock_least_nk(const dsm_sim* s) {
   const double b = (double)s->P.beta;
   if (b > 4.0) return 0.0;
-  if (!s->corr) return std::max(75.0, 85.0 / b);
+  if (!s->corr) return std::max(60.0, 65.0 / b);
   if (b < 0.4) return 0.0;
   return std::max({s->ck == 2 || b > 1.0 ? 175.0 : 150.0, 75.0 * b, std::min(230.0, 120.0 / b)});
 }
@@ -261,22 +262,24 @@ static bool prefer_lock(const dsm_sim* s) {
 // chain in and out at several times the cost of a tile (a service warp does it, two
 // for up to 16 slots; the vectors go back to strand order) and has to earn that by
 // its events.  Measured crossings, 8192 to 65536 chains (more chains, later):
-//   none  beta 1    N_K 87 230 to 380, 100 160 to 220, 150 100 to 170, 200 60 to 150, 300 95
-//         beta 0.5  N_K 170 380 to 600, 240 190, 463 80   beta 2  N_K 75 280, 150 170 to 320, 300 100
-//         beta 4    N_K 75 390 to 750, 150 290 to 450, 300 340
+//   none  beta 1    N_K 67 350 to 800, 75 220 to 330, 100 120, 150 140, 200 110 to 130, 300 50
+//         beta 0.5  N_K 150 170 to 270, 200 140 to 250, 300 80, 463 75
+//         beta 2    N_K 60 180 to 230, 100 130 to 145, 200 140
+//         beta 4    N_K 60 270 to 350, 100 220, 300 170 to 190
 //   G(t)  beta 1    N_K 150 260 to 600, 200 180 to 500, 300 130 to 180
 //         beta 0.5  N_K 240 340 to 380, 300 160 to 240, 463 25 to 35 (8 tiles per SM)
 //         beta 2    N_K 175 390 to 550, 300 105 to 130   beta 4  N_K 300 500 to 700
-//   MSD   beta 1    N_K 175 600, 200 210 to 700, 300 140 to 200, which with tiles of
-//         16 lanes where 32 are faster is 50
+//   MSD   beta 1    N_K 175 600, 200 210 to 700, 300 140 to 200; against tiles of 16
+//         lanes where 32 are faster (default_schedule) 50, none at 8 tiles per SM
 // Below them the start of a window counts: 0.1 tau of 16384 chains of N_K = 200, G(t),
 // 0.15 ms in tiles and 0.34 in lockstep, 1 tau 0.47 and 0.68, 5 tau 1.78 and 1.73.
 static double lock_least_events(const dsm_sim* s, int tile_lanes, int tiles_per_sm) {
   const double x = (double)s->P.nk / lock_least_nk(s);
-  if (!s->corr) return std::max(100.0, 350.0 * std::max(1.0, 0.5 * (double)s->P.beta) / x);
-  if (s->ck == 2 && tile_lanes != 16) return 50.0;
-  const double r = std::min(1.0, tiles_per_sm / 16.0);
-  return std::max(30.0, 600.0 * r * r / (x * x));
+  const bool one = tile_lanes != 16;  // one chain per warp, for long chains
+  if (!s->corr) return std::max(1.0, 0.5 * (double)s->P.beta) * std::max(one ? 70.0 : 110.0, 300.0 / (x * x));
+  if (s->ck == 2 && one) return tiles_per_sm < 16 ? 0.0 : 50.0;
+  const double r = one ? tiles_per_sm / 16.0 : 1.0;
+  return std::max(30.0, (one ? 420.0 : 600.0) * r * r / (x * x));
 }
 
 int dsm::sim_setup(dsm_sim* s) {
@@ -476,10 +479,12 @@ static void fit_block(bool flow, LaunchCfg& cfg, int optin) {
   while (cfg.warps_per_block > 1 && step_block_smem(flow, cfg) > (size_t)optin) cfg.warps_per_block /= 2;
 }
 
-// Slots per block of a lockstep launch over n chains: as many as fit 6 blocks
+// Slots per block of a lockstep launch over n chains: as many as fit 5 blocks
 // per SM when that is a full block (and the kernel has a build for it), else as
 // many as fit 4; with few chains no more than spread them over all SMs.  Returns
-// the blocks per SM the choice is made for (0: not a lockstep launch).
+// the blocks per SM the choice is made for (0: not a lockstep launch).  (A build for
+// 6 blocks spills at its 80 registers: 16384 chains, 30 tau, N_K = 100 4.7 ms against
+// 4.1, N_K = 170, beta = 0.5 9.6 and 8.5; 12000 of N_K = 120 4.6 and 3.3.)
 static int plan_lock(const dsm_sim* s, LaunchCfg& c, long long n) {
   c.tiles = 0;
   if (!c.lock || s->flow || lock_lanes(c.slot_cap) == 0) return 0;
@@ -492,7 +497,7 @@ static int plan_lock(const dsm_sim* s, LaunchCfg& c, long long n) {
     while (t > 0 && (lock_block_bytes(c.slot_cap, t) + reserved) * blocks > (size_t)sm_bytes) --t;
     return t;
   };
-  int bps = 6, t = fits(6);
+  int bps = 5, t = fits(5);
   if (t < most || s->ck != 0) {
     bps = 4;
     t = fits(4);

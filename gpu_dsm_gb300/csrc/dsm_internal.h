@@ -134,7 +134,7 @@ struct LaunchCfg {
 __host__ __device__ size_t step_slot_bytes(int slot_cap, int pmax);
 // lockstep kernel (dsm_lockstep.cu): lanes per chain at a slot size (0: not built
 // for it), shared memory of a block of `tiles` slots, and the kernel of a
-// correlator kind (hi: the build for 6 blocks per SM)
+// correlator kind (hi: the build for 5 blocks per SM)
 int lock_lanes(int slot_cap);
 bool lock_slices(int slot_cap);  // launches in time slices pay for slots of this size
 size_t lock_block_bytes(int slot_cap, int tiles);

@@ -514,7 +514,7 @@ __device__ __forceinline__ uint32_t lock_struct(const EnsDev& E, const LSlot& sl
     // lanes 0 and 1 a pair of normal deviates each, lane 2 the lifetime's power
     const uint32_t gx = wshfl(w.x, 1), gy = wshfl(w.y, 1), gz = wshfl(w.z, 1), gw = wshfl(w.w, 1);
     // (one N_K, no GEX background: the ensemble's own partner law)
-    const PcdDev& pp = E.pcd;
+    const PcdDev pp = E.pcd;
     const float pA = cdc ? pp.Adt_ : pp.At_, pD = cdc ? pp.Ddt_ : pp.Dt_, pC = cdc ? pp.Cdt_ : pp.Ct_;
     const float pB = cdc ? pp.Bdt_ : pp.one_minus_g;
     const float u = u01(w2);
@@ -1270,7 +1270,7 @@ static void* lock_pick(const LockShape& f) {
 }
 void* lock_kernel(int ck, int slot_cap, bool hi) {
   const LockShape f = lock_shape(slot_cap);
-  if (hi) return ck == 0 ? lock_pick<0, 6>(f) : nullptr;
+  if (hi) return ck == 0 ? lock_pick<0, 5>(f) : nullptr;
   return ck == 0 ? lock_pick<0, 4>(f) : ck == 2 ? lock_pick<2, 4>(f) : lock_pick<1, 4>(f);
 }
 
