@@ -4,6 +4,7 @@
 // layout.  Replaces the process-global ensemble / call-block machinery of the
 // reference (common/ensemble.cu, common/ensemble_call_block.cu).
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdint>
@@ -130,6 +131,7 @@ static int small_schedule(dsm_sim* s);
 static void series_free(dsm_sim* s);
 static int enqueue_readback(dsm_sim* s);
 static int window_collect(dsm_sim* s, uint64_t* events);
+static void flight_end(dsm_sim* s);
 
 static bool is_flow(const float* k) {
   for (int q = 0; q < 9; ++q) if (k[q] != 0.0f) return true;
@@ -780,6 +782,7 @@ int dsm::plan_carve(dsm_sim* s, const SizeClass& B, const SizeClass& M, const Si
 extern "C" void dsm_destroy(dsm_sim* s) {
   if (!s) return;
   if (s->st) cudaStreamSynchronize(s->st);
+  flight_end(s);
   if (s->st) series_free(s);
   if (s->side) cudaStreamSynchronize(s->side);
   if (s->side2) cudaStreamSynchronize(s->side2);
@@ -879,10 +882,51 @@ static int default_schedule(dsm_sim* s) {
   return rl;
 }
 
+// Chains of the handles' launches that are under way on a device (not of
+// dsm_advance_batch, which sees all its ensembles), and of all launches so far, so that
+// small ensembles that run side by side share the SMs two chains per warp
+// (small_schedule).  A hint: results do not depend on it.
+struct Flights {
+  std::atomic<long long> now{0}, begun{0};
+};
+static Flights& flights(const dsm_sim* s) {
+  static Flights f[64];
+  return f[s->P.device & 63];
+}
+// Whether the chains of s and those beside it, now and during its last launch, are at
+// most `most`
+static bool flight_fits(const dsm_sim* s, long long most) {
+  const long long n = s->P.n_chains, now = flights(s).now.load() - (s->flying ? n : 0);
+  return n + std::max(now, s->beside) <= most;
+}
+static void flight_begin(dsm_sim* s) {
+  Flights& f = flights(s);
+  const long long n = s->P.n_chains;
+  s->beside = s->flying ? f.now.load() - n : f.now.fetch_add(n);
+  s->flying = true;
+  s->flight = f.begun.fetch_add(n) + n;
+}
+static void flight_end(dsm_sim* s) {
+  if (!s->flying) return;
+  Flights& f = flights(s);
+  s->flying = false;
+  s->beside += f.begun.load() - s->flight;
+  f.now.fetch_sub(s->P.n_chains);
+}
+
 // The plan of a launch of windows of dt_tau (or up to step_limit events per chain):
 // a default lockstep ensemble runs tiles where the chains do fewer than lock_events
 // events.  The sums and the state are the same.
+static void swap_plans(dsm_sim* s) {
+  std::swap(s->cfg, s->other.cfg);
+  s->classes.swap(s->other.classes);
+  std::swap(s->cleanup, s->other.cleanup);
+  std::swap(s->grid, s->other.grid);
+  std::swap(s->blocks_per_sm, s->other.blocks_per_sm);
+  std::swap(s->sub_max, s->other.sub_max);
+}
 static void choose_plan(dsm_sim* s, double dt_tau, int64_t step_limit) {
+  if (s->slot16 > 0 && (s->cfg.lanes == 32) != flight_fits(s, 24ll * s->sm_count)) swap_plans(s);
   if (s->lock_events <= 0.0) return;
   double ev = kEventsPerTau * (double)s->P.nk * std::max(0.0, dt_tau);
   if (step_limit >= 0) {
@@ -890,13 +934,7 @@ static void choose_plan(dsm_sim* s, double dt_tau, int64_t step_limit) {
     const double left = (double)step_limit - (double)(s->events_total - s->events_base) / (double)s->P.n_chains;
     ev = dt_tau > 0.0 ? std::min(ev, left) : left;
   }
-  if ((ev >= s->lock_events) == s->cfg.lock) return;
-  std::swap(s->cfg, s->other.cfg);
-  s->classes.swap(s->other.classes);
-  std::swap(s->cleanup, s->other.cleanup);
-  std::swap(s->grid, s->other.grid);
-  std::swap(s->blocks_per_sm, s->other.blocks_per_sm);
-  std::swap(s->sub_max, s->other.sub_max);
+  if ((ev >= s->lock_events) != s->cfg.lock) swap_plans(s);
 }
 
 // Blocks per SM of one launch with one chain per warp and full-capacity slots,
@@ -915,7 +953,10 @@ static int one_per_warp(bool flow, int ck, int cap, int pmax, int optin, LaunchC
 // 0.429, 0.644 and 0.564.  Not where the 16-lane plan is one of 4 blocks per SM
 // (G(t) of long chains, whose larger register budget leaves little: 3648 chains of
 // N_K = 100 0.62 either way), not for MSD (as in poly_schedule), and not for
-// ensembles that share the GPU with others.
+// ensembles that share the GPU with others: not in the server, and, launch by launch
+// (choose_plan), not beside launches of other handles with too many chains (12 tau of 8 ensembles of 3000
+// chains of N_K = 50 at once, without G(t): 1.98 ms one per warp, 1.85 two per warp,
+// in shear 2.69 and 2.39; 20 tau of N_K = 100 5.37 and 4.43).
 static int small_schedule(dsm_sim* s) {
   const dsm_params& P = s->P;
   if (P.lanes_per_chain != 0 || s->shared || s->ck == 2 || s->poly || s->cfg.lock || s->cfg.lanes != 16 || s->blocks_per_sm < 5 ||
@@ -927,6 +968,7 @@ static int small_schedule(dsm_sim* s) {
   const int bps = one_per_warp(s->flow, s->ck, s->cap, s->cfg.pmax, optin, c);
   if (P.n_chains > (long long)bps * s->sm_count * step_tiles(s->flow, c)) return DSM_OK;
   s->slot16 = s->classes.empty() ? s->cap : s->classes.back().cfg.slot_cap;
+  s->other = StepPlan{s->cfg, s->classes, s->cleanup, s->grid, s->blocks_per_sm, s->sub_max};
   s->cfg.lanes = 32;
   return plan_single(s);
 }
@@ -1387,6 +1429,7 @@ int dsm::sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit) {
   E.t_end_ticks = (int64_t)std::llrint(t_end * TICKS);
   s->t_window = t_end;
   choose_plan(s, t_end - s->t_done, step_limit);
+  flight_begin(s);
   E.step_limit = step_limit < 0 ? INT64_MAX : step_limit;
   E.watchdog_events = window_watchdog(s, t_end - s->t_done);
   E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
@@ -1501,7 +1544,8 @@ static int series_prepare(dsm_sim* s, int n, cudaGraphExec_t* exec) {
     s->ser_version = s->sched_version;
   }
   if (!exec) return DSM_OK;  // buffers only (windows issued directly)
-  const int key = 2 * n + (s->cfg.lock ? 1 : 0);  // (choose_plan does not change the schedule's version)
+  // (choose_plan does not change the schedule's version)
+  const int key = 4 * n + (s->cfg.lock ? 1 : s->cfg.lanes == 32 ? 2 : 0);
   for (auto& g : s->ser_graphs)
     if (g.first == key) { *exec = g.second; return DSM_OK; }
   cudaGraphExec_t e = nullptr;
@@ -1526,6 +1570,7 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   // did not), while a few launches per window cost nothing next to windows of
   // seconds.
   choose_plan(s, (ends[n - 1] - s->t_done) / n, -1);
+  flight_begin(s);
   const bool direct = !s->classes.empty();
   cudaGraphExec_t exec = nullptr;
   int rc = series_prepare(s, n, direct ? nullptr : &exec);
@@ -1588,6 +1633,7 @@ static void stress_out(const double* r, dsm_stress_plus* o) {
 }
 
 static int series_collect(dsm_sim* s, dsm_stress_plus* out, uint64_t* events) {
+  flight_end(s);
   CK(cudaGetLastError());
   const int n = s->ser_n;
   const double* h_out = ser_out_h(s);
@@ -1725,6 +1771,7 @@ static int enqueue_readback(dsm_sim* s) {
 
 // Host bookkeeping of a completed window (its readback has landed)
 static int window_collect(dsm_sim* s, uint64_t* events) {
+  flight_end(s);
   CK(cudaGetLastError());
   const unsigned long long* cnt = s->hw->cnt;
   const int rc = launch_status(s, s->hw->status);

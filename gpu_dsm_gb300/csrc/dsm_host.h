@@ -153,6 +153,10 @@ struct dsm_sim {
   // chain than lock_events (0: one plan); choose_plan swaps the two
   double lock_events = 0.0;
   dsm::StepPlan other;
+  // a small_schedule plan has its two-per-warp form there; chains of other handles'
+  // launches beside this handle's last one (Flights)
+  bool flying = false;
+  long long beside = 0, flight = 0;
   uint64_t events_base = 0;  // events_total when the chains were set
   bool by_default = false;    // monodisperse: the plan is the default one, not one that was asked for
   // one chain per warp because all chains are resident so (small_schedule): the
