@@ -177,7 +177,9 @@ extern "C" int dsm_checkpoint_load(dsm_sim* s, const char* path) {
   if (total != h.payload_bytes || ck != h.checksum) return fail(s, DSM_ERR_INVALID, "checkpoint checksum mismatch");
   // the chains' N_K must be this ensemble's (polydisperse ensembles keep them per chain)
   const ChainState* cs = (const ChainState*)host[0].data();
+  double t_chains = 0.0;
   for (int64_t i = 0; i < h.n_chains; ++i) {
+    t_chains += (double)cs[i].T / dsm::TICKS / (double)h.n_chains;
     if (cs[i].nk != s->nk_chain[(size_t)i]) return differ("per-chain N_K");
     if (cs[i].Z < 1 || cs[i].Z > s->cap) return fail(s, DSM_ERR_INVALID, "corrupt checkpoint (Z out of range)");
   }
@@ -192,5 +194,6 @@ extern "C" int dsm_checkpoint_load(dsm_sim* s, const char* path) {
   s->t_window = h.t_done;
   s->events_total = h.events_total;
   s->events_base = 0;
+  s->t_chains = t_chains;
   return DSM_OK;
 }

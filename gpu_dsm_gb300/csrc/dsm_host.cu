@@ -914,9 +914,16 @@ static void flight_end(dsm_sim* s) {
   f.now.fetch_sub(s->P.n_chains);
 }
 
-// The plan of a launch of windows of dt_tau (or up to step_limit events per chain):
-// a default lockstep ensemble runs tiles where the chains do fewer than lock_events
-// events.  The sums and the state are the same.
+// The chains' mean time after a launch of `events` events to t_end: t_end, or, when it
+// was cut short, what the events amount to
+static void chains_at(dsm_sim* s, double t_end, unsigned long long events, bool cut) {
+  const double t = s->t_chains + (double)events / (kEventsPerTau * (double)s->P.nk * (double)s->P.n_chains);
+  s->t_chains = cut ? std::min(t, std::max(s->t_chains, t_end)) : std::max(s->t_chains, t_end);
+}
+
+// The plan of a launch of windows of dt_tau from the chains' time (or up to step_limit
+// events per chain): a default lockstep ensemble runs tiles where the chains do fewer
+// than lock_events events.  The sums and the state are the same.
 static void swap_plans(dsm_sim* s) {
   std::swap(s->cfg, s->other.cfg);
   s->classes.swap(s->other.classes);
@@ -929,11 +936,8 @@ static void choose_plan(dsm_sim* s, double dt_tau, int64_t step_limit) {
   if (s->slot16 > 0 && (s->cfg.lanes == 32) != flight_fits(s, 24ll * s->sm_count)) swap_plans(s);
   if (s->lock_events <= 0.0) return;
   double ev = kEventsPerTau * (double)s->P.nk * std::max(0.0, dt_tau);
-  if (step_limit >= 0) {
-    // (after an event-limited launch the chains are behind the handle's time)
-    const double left = (double)step_limit - (double)(s->events_total - s->events_base) / (double)s->P.n_chains;
-    ev = dt_tau > 0.0 ? std::min(ev, left) : left;
-  }
+  if (step_limit >= 0)
+    ev = std::min(ev, (double)step_limit - (double)(s->events_total - s->events_base) / (double)s->P.n_chains);
   if ((ev >= s->lock_events) != s->cfg.lock) swap_plans(s);
 }
 
@@ -1215,12 +1219,19 @@ extern "C" int dsm_init_equilibrium(dsm_sim* s) {
   if (rc) return rc;
   CK(launch_init(s->d_ens, s->h, s->cap, s->st));
   CK(cudaStreamSynchronize(s->st));
+  s->t_chains = 0.0;
   s->lost = false;
   s->events_base = s->events_total;
   return DSM_OK;
 }
 
 // ------------------------------------------------------------------ state transfer
+static double mean_time(const std::vector<ChainState>& cs) {
+  double t = 0.0;
+  for (const ChainState& c : cs) t += (double)c.T;
+  return t / TICKS / (double)cs.size();
+}
+
 extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm_float4* QN, const float* tau) {
   const dsm::NvtxRange nvtx_range("dsm_set_chains");
   if (!s || !s->ready || !heads || !QN || !tau) return DSM_ERR_INVALID;
@@ -1268,6 +1279,7 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
   int rc = reset_corr(s);
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
+  s->t_chains = mean_time(cs);
   s->lost = false;
   s->events_base = s->events_total;
   return DSM_OK;
@@ -1332,6 +1344,7 @@ extern "C" int dsm_set_ext(dsm_sim* s, const int64_t* T, const uint64_t* steps, 
   }
   CK(cudaMemcpyAsync(s->d_cs, cs.data(), n * sizeof(ChainState), cudaMemcpyHostToDevice, s->st));
   CK(cudaStreamSynchronize(s->st));
+  s->t_chains = mean_time(cs);
   return DSM_OK;
 }
 
@@ -1428,12 +1441,12 @@ int dsm::sim_launch_window(dsm_sim* s, double t_end, int64_t step_limit) {
   EnsDev& E = s->h;
   E.t_end_ticks = (int64_t)std::llrint(t_end * TICKS);
   s->t_window = t_end;
-  choose_plan(s, t_end - s->t_done, step_limit);
+  choose_plan(s, t_end - s->t_chains, step_limit);
   flight_begin(s);
   E.step_limit = step_limit < 0 ? INT64_MAX : step_limit;
   E.watchdog_events = window_watchdog(s, t_end - s->t_done);
-  E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
-  E.subs = launch_slices(s, t_end - s->t_done, step_limit);
+  E.t_begin_ticks = (int64_t)std::llrint(s->t_chains * TICKS);
+  E.subs = launch_slices(s, t_end - s->t_chains, step_limit);
   CK(cudaMemcpyAsync(s->d_ens, &E, sizeof(EnsDev), cudaMemcpyHostToDevice, s->st));
   CK(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->st));
   CK(cudaMemsetAsync(s->d_counters, 0, 4 * sizeof(unsigned long long), s->st));
@@ -1569,7 +1582,7 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   // 10-20 % slower on the 262144-chain log-normal melt (a graph of one window
   // did not), while a few launches per window cost nothing next to windows of
   // seconds.
-  choose_plan(s, (ends[n - 1] - s->t_done) / n, -1);
+  choose_plan(s, (ends[n - 1] - s->t_chains) / n, -1);
   flight_begin(s);
   const bool direct = !s->classes.empty();
   cudaGraphExec_t exec = nullptr;
@@ -1577,18 +1590,18 @@ static int series_start(dsm_sim* s, const double* ends, int n) {
   if (rc != DSM_OK) return rc;
   long long* h_win = ser_win_h(s);
   t_prev = s->t_done;
-  double shortest = ends[n - 1] - t_prev;
+  double shortest = ends[0] - s->t_chains;
   for (int w = 0; w < n; ++w) {
     h_win[w] = (long long)std::llrint(ends[w] * TICKS);  // as dsm_advance(ends[w])
     h_win[s->ser_cap + w] = (long long)window_watchdog(s, ends[w] - t_prev);
-    shortest = std::min(shortest, ends[w] - t_prev);
+    if (w > 0) shortest = std::min(shortest, ends[w] - t_prev);
     t_prev = ends[w];
   }
   s->t_window = t_prev;
   s->ser_n = n;
   EnsDev& E = s->h;
   E.step_limit = INT64_MAX;
-  E.t_begin_ticks = (int64_t)std::llrint(s->t_done * TICKS);
+  E.t_begin_ticks = (int64_t)std::llrint(s->t_chains * TICKS);
   E.subs = launch_slices(s, shortest, -1);
   CK(cudaMemcpyAsync(s->d_ens, &E, sizeof(EnsDev), cudaMemcpyHostToDevice, s->st));
   if (direct) {
@@ -1644,6 +1657,7 @@ static int series_collect(dsm_sim* s, dsm_stress_plus* out, uint64_t* events) {
   s->events_total += ev;
   s->last_events = ev;
   s->t_done = s->t_window;
+  chains_at(s, s->t_window, ev, rc == DSM_ABORTED);
   CK(cudaEventElapsedTime(&s->last_kernel_ms, s->ev0, s->ev1));
   if (s->flow) {
     for (int q = 0; q < 9; ++q) s->hw->red[q] = h_out[9 * (n - 1) + q];
@@ -1779,6 +1793,7 @@ static int window_collect(dsm_sim* s, uint64_t* events) {
   if (events) *events = cnt[0];
   s->events_total += cnt[0];
   s->t_done = std::max(s->t_done, s->t_window);
+  chains_at(s, s->t_window, cnt[0], rc == DSM_ABORTED || s->h.step_limit != INT64_MAX);
   s->last_events = cnt[0];
   CK(cudaEventElapsedTime(&s->last_kernel_ms, s->ev0, s->ev1));
   return rc;
@@ -1962,7 +1977,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
   auto cap_class = [](int cap) { int c = 16; while (c < cap) c <<= 1; return c; };
   std::vector<Group> groups;
   for (int i = 0; i < n; ++i) {
-    choose_plan(sims[i], t_end[i] - sims[i]->t_done, step_limit ? step_limit[i] : -1);
+    choose_plan(sims[i], t_end[i] - sims[i]->t_chains, step_limit ? step_limit[i] : -1);
     const bool fl = sims[i]->flow;
     const int co = sims[i]->ck;
     const int cc = cap_class(sims[i]->cap), cp = co ? sims[i]->cp : 0;
@@ -2140,6 +2155,7 @@ extern "C" int dsm_advance_batch(dsm_sim** sims, int32_t n, const double* t_end,
     sims[i]->events_total += cnt[0];
     sims[i]->last_events = cnt[0];
     sims[i]->t_done = std::max(sims[i]->t_done, sims[i]->t_window);
+    chains_at(sims[i], sims[i]->t_window, cnt[0], sims[i]->h.step_limit != INT64_MAX);
   }
   if (status != DSM_OK && !s->lost) fail(s, status, "a wait between warps ran out; an ensemble of the batch is lost");
   return status;

@@ -157,6 +157,9 @@ struct dsm_sim {
   // launches beside this handle's last one (Flights)
   bool flying = false;
   long long beside = 0, flight = 0;
+  // mean time of the chains, which t_done (the latest window's end) is not after they
+  // are set, or when a launch was cut short
+  double t_chains = 0.0;
   uint64_t events_base = 0;  // events_total when the chains were set
   bool by_default = false;    // monodisperse: the plan is the default one, not one that was asked for
   // one chain per warp because all chains are resident so (small_schedule): the

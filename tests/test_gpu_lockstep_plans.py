@@ -117,12 +117,22 @@ def test_short_and_long_windows(dsm_mod, kw):
         assert dsm_mod.advance_batch([a], t)[0] == b.advance(t)
         assert a.step_kernel()["lockstep"] == lock
     done = int(b.get_ext()["step"].mean())
-    for limit, lock in ((done + 40, False), (done + 1500, True)):
+    for limit, lock in ((done + 40, False), (done + 1500, True), (done + 1540, False)):
         assert a.advance(1.0e6, step_limit=limit) == b.advance(1.0e6, step_limit=limit)
         assert a.step_kernel()["lockstep"] == lock
     assert_bitexact(gpu_state(a), gpu_state(b), what="short and long windows")
     if "eq_type" in kw:
         assert np.array_equal(a.gt_raw()[0], b.gt_raw()[0]) and np.array_equal(a.gt_raw()[1], b.gt_raw()[1])
+    # chains set anew begin at their own time, not at the handle's
+    heads, qn, tau = a.get_chains()
+    heads["time"] = 0.0
+    for _ in range(2):
+        for x in (a, b):
+            x.set_chains(heads, qn, tau)
+        for t, lock in ((30.0, True), (30.5, False), (70.5, True)):
+            assert a.advance(t) == b.advance(t)
+            assert a.step_kernel()["lockstep"] == lock
+    assert_bitexact(gpu_state(a), gpu_state(b), what="chains set anew")
 
 
 def test_slices_of_a_launch(dsm_mod):
@@ -132,6 +142,11 @@ def test_slices_of_a_launch(dsm_mod):
     assert e.step_kernel() == {"lockstep": True, "lanes": 8, "slot": e.step_kernel()["slot"], "slices": 4}
     e.advance(65.0)  # some 600 events per chain
     assert e.step_kernel()["lockstep"] and e.step_kernel()["slices"] == 1
+    heads, qn, tau = e.get_chains()
+    heads["time"] = 0.0
+    e.set_chains(heads, qn, tau)
+    e.advance(55.0)
+    assert e.step_kernel()["slices"] == 4
 
 
 @pytest.mark.parametrize("ends,slices", [((80.0, 81.0, 161.0), 1), ((80.0, 160.0, 240.0), 4)], ids=str)
