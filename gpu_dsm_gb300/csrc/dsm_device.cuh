@@ -1,5 +1,5 @@
 // Device functions shared by the step kernels (dsm_kernels.cu: one or two
-// chains per warp; dsm_lockstep.cu: four chains per warp in lockstep): rate
+// chains per warp; dsm_lockstep.cu: eight or four chains per warp in lockstep): rate
 // quantisation, random words, lifetime samplers, sliding rates, the split of a
 // created strand and the correlator's level-0 counters.
 #pragma once

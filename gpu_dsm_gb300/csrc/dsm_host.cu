@@ -986,8 +986,8 @@ static void small_schedule_end(dsm_sim* s) {
 // Per-chain N_K.  One chain per warp has the lower latency, two per warp (16 lanes,
 // with a middle class of one per warp for the chains that outgrow its slot) the
 // higher throughput, which counts when the whole work at its 1.9e9 events/s lasts
-// longer than the longest chain at 2.2 us per event: sum N_K above 4100 times the
-// largest N_K.  A middle class between a hundredth of the chains and two full
+// longer than the longest chain in company at 2.2 us per event (1.0 us alone): sum
+// N_K above 4100 times the largest N_K.  A middle class between a hundredth of the chains and two full
 // rounds of its slots holds the other one up.  20 tau of G(t), 32 and 16 lanes:
 // 32768 chains, mean N_K 150, PDI 1.5 (6060 in the middle class) 12.4 and 11.2 ms;
 // 16384, 100, 1.1 (93) 4.8 and 3.5; 32768, 50, 1.1 (none) 5.0 and 4.2; but 32768,

@@ -39,7 +39,6 @@ struct ChainState {
 };
 static_assert(sizeof(ChainState) == 64, "ChainState layout");
 
-// Everything one kernel needs to know about one ensemble (device copy).
 // A chain of a launch in time slices
 struct __align__(16) Slice {
   unsigned long long step0;  // event counter at the start of the launch
@@ -48,6 +47,7 @@ struct __align__(16) Slice {
 };
 constexpr unsigned kMoved = 0xffffffffu;
 
+// Everything one kernel needs to know about one ensemble (device copy).
 struct EnsDev {
   int32_t n_chains, cap, nk, cd_flag;
   int32_t flow, s0, poly, corr_type;

@@ -3,8 +3,8 @@
 // Most kMC events are slides (N_K = 200: 94 %).  A slide warp runs 8 chains with
 // 4 lanes each (4 chains with 8 lanes where slots are long) and does one event of
 // all of them per round, every lane on the same instruction, so that one
-// instruction stream serves 8 chains: 174 warp instructions per event at
-// N_K = 200 without G(t) (201 with it), against 301 of the 16-lane tiles of
+// instruction stream serves 8 chains: 172 warp instructions per event at
+// N_K = 200 without G(t) (198 with it), against 301 of the 16-lane tiles of
 // dsm_kernels.cu.  A tile's rare paths (a creation runs 4600 cycles) would hold
 // up the whole warp here; so whatever is not a slide -- creations and
 // destructions, samples, the end of a window, the next chain, full rate passes --
@@ -15,7 +15,8 @@
 // and the instruction cache.  An SM fetches up to 32 KB of code at one
 // instruction per cycle and the next 96 KB at 2.7 cycles each; the slide loop
 // (12 KB), the creations and destructions (10 KB) and the samples just about
-// fill it (a quarter of the stalls are waits for instructions).  Hence one copy
+// fill it (with G(t) a quarter of the stalls are waits for instructions, 2.1 warps
+// per issue; without, 0.7).  Hence one copy
 // of the random words, of the full rate pass and of the correlator (which takes
 // kCorrBuf samples at a time), rare code kept rolled, and two service warps per
 // two slide warps: with three or four, more code is in flight at once and the
@@ -25,7 +26,7 @@
 // creations, destructions and samples read them, in the service warps, from L2),
 // which leaves 24 bytes per strand: 60 chains per SM at N_K = 200 instead of 32.
 // Four lanes per chain against eight at that size: 3.87e9 against 3.17e9 events/s
-// without G(t).
+// without G(t).  4.10e9 now without G(t), 3.15e9 with it (500 tau).
 //
 // Trajectories, samples and sums are those of dsm_kernels.cu bit for bit.
 #include <cstdint>
@@ -40,8 +41,6 @@ namespace dsm {
 
 namespace {
 
-// A slide warp runs 32 / G chains with G lanes each; the pick has 4 sub-chunks of
-// SB pairs per lane
 // What a slide warp asks a service warp for
 enum : int { RQ_STRUCT = 1, RQ_FULL = 4, RQ_TIME = 8, RQ_STALL = 16, RQ_LOAD = 32 };
 
@@ -918,6 +917,8 @@ __device__ __noinline__ bool lock_moved(const EnsDev* ens, const unsigned int* w
   return wshfl(moved, 0) != 0;
 }
 
+// A slide warp runs 32 / G chains with G lanes each; the pick has 4 sub-chunks of
+// SB pairs per lane.
 template <int CK, int G, int SB, int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_lock(const EnsDev* __restrict__ ens, int n_ens,
                                                   const long long* __restrict__ prefix, long long total,
