@@ -12,6 +12,7 @@
 #include <cstring>
 #include <fstream>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1226,12 +1227,6 @@ extern "C" int dsm_init_equilibrium(dsm_sim* s) {
 }
 
 // ------------------------------------------------------------------ state transfer
-static double mean_time(const std::vector<ChainState>& cs) {
-  double t = 0.0;
-  for (const ChainState& c : cs) t += (double)c.T;
-  return t / TICKS / (double)cs.size();
-}
-
 extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm_float4* QN, const float* tau) {
   const dsm::NvtxRange nvtx_range("dsm_set_chains");
   if (!s || !s->ready || !heads || !QN || !tau) return DSM_ERR_INVALID;
@@ -1242,8 +1237,10 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
   const size_t nt = std::max<size_t>(1, std::min<size_t>({16, std::thread::hardware_concurrency(), n / 4096 + 1}));
   std::vector<size_t> bad(nt, n);
   std::vector<int> why(nt, 0);
+  std::vector<double> time(nt, 0.0);
   auto work = [&](size_t r) {
     const size_t i0 = n * r / nt, i1 = n * (r + 1) / nt;
+    double t = 0.0;
     for (size_t i = i0; i < i1; ++i) {
       const int Z = heads[i].Z;
       int code = 0;
@@ -1261,7 +1258,9 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
       c.Z = Z; c.stall = heads[i].stall_flag; c.S = s->h.s0; c.dt_prev = 0.f;
       c.T = (int64_t)std::llrint((double)heads[i].time * TICKS);
       c.step = 0; c.hash = 0xCBF29CE484222325ull; c.k_next = 0; c.nk = s->nk_chain[i];
+      t += (double)c.T;
     }
+    time[r] = t;
   };
   std::vector<std::thread> pool;
   for (size_t r = 1; r < nt; ++r) pool.emplace_back(work, r);
@@ -1279,7 +1278,7 @@ extern "C" int dsm_set_chains(dsm_sim* s, const dsm_chain_head* heads, const dsm
   int rc = reset_corr(s);
   if (rc) return rc;
   CK(cudaStreamSynchronize(s->st));
-  s->t_chains = mean_time(cs);
+  s->t_chains = std::accumulate(time.begin(), time.end(), 0.0) / TICKS / (double)n;
   s->lost = false;
   s->events_base = s->events_total;
   return DSM_OK;
@@ -1344,7 +1343,10 @@ extern "C" int dsm_set_ext(dsm_sim* s, const int64_t* T, const uint64_t* steps, 
   }
   CK(cudaMemcpyAsync(s->d_cs, cs.data(), n * sizeof(ChainState), cudaMemcpyHostToDevice, s->st));
   CK(cudaStreamSynchronize(s->st));
-  s->t_chains = mean_time(cs);
+  if (T) {
+    s->t_chains = 0.0;
+    for (size_t i = 0; i < n; ++i) s->t_chains += (double)T[i] / TICKS / (double)n;
+  }
   return DSM_OK;
 }
 
