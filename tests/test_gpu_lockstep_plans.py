@@ -229,18 +229,21 @@ def test_abort_between_two_slices(dsm_mod):
     a, b = dsm_mod.Ensemble(**kw), dsm_mod.Ensemble(lanes_per_chain=16, **kw)
     for x in (a, b):
         x.init_equilibrium()
+    begin, end = 300.0, 3300.0
+    assert a.advance(begin) == b.advance(begin)
+    a_window = a.last_window()["kernel_ms"] * 1.0e-3
     flag = np.zeros(1, np.int32)
-    timer = threading.Timer(0.25, lambda: flag.__setitem__(0, 1))
+    timer = threading.Timer(0.45 * a_window * (end - begin) / begin, lambda: flag.__setitem__(0, 1))
     timer.start()
-    end = 3000.0
     assert a.advance(end, abort=flag) == -1
     timer.join()
     k = a.step_kernel()["slices"]
     assert k > 1
     T = a.get_ext()["T"] / TICKS
-    done = np.floor(T / (end / k) + 1e-9).astype(int)  # slices each chain has finished
+    piece = (end - begin) / k
+    done = np.floor((T - begin) / piece + 1e-9).astype(int)  # slices each chain has finished
     assert done.max() >= 1 and T.min() < end
-    stopped = (done >= 1) & (done < k) & (T - done * (end / k) < 1.0)  # just past a slice's end
+    stopped = (done >= 1) & (done < k) & (T - begin - done * piece < 1.0)  # just past a slice's end
     assert stopped.sum() > 50
     assert a.advance(end) != -1
     b.advance(end)
